@@ -251,8 +251,10 @@ b200fmm_status b200fmm_create(const b200fmm_config *cfg, b200fmm_handle *out) {
     st = compress_sym_operators(*c);
     if (st == B200FMM_OK && cfg->precision == B200FMM_FP64) st = upload_sym_operators(*c);
   }
-  if (st == B200FMM_OK && cfg->kernel != B200FMM_CHEB_SYM && cfg->precision == B200FMM_FP64)
-    st = build_dense_operators(*c);
+  if (st == B200FMM_OK && cfg->kernel != B200FMM_CHEB_SYM && cfg->precision == B200FMM_FP64) {
+    st = build_dense_operators(*c, (c->nn + 7) & ~7);
+    if (st == B200FMM_OK) st = dense64_prepare(*c);
+  }
   if (st == B200FMM_OK && cfg->precision == B200FMM_MIXED) st = tc_init(*c);
   if (st != B200FMM_OK) {
     destroy_context(c);
@@ -321,8 +323,13 @@ b200fmm_status b200fmm_set_particles(b200fmm_handle h, long long n, const double
   if (st != B200FMM_OK) return st;
   B200_CHECK(zero_state(c));  // a new tree starts from zero expansions and results
   c.state_zero = true;
+  // the FP64 M2L's per-tree tables for dense operators need a count from the device: it travels under the wait below
+  const bool dense64 = c.cfg.precision == B200FMM_FP64 && c.cfg.kernel != B200FMM_CHEB_SYM;
+  int *dense_first = (int *)(c.h_pinned + 64);
+  if (dense64) B200_CHECK(dense64_tree_counts(c, dense_first));
   B200_CUDA(cudaEventRecord(c.ev[15], c.stream));
   B200_CUDA(cudaEventSynchronize(c.ev[15]));
+  if (dense64) B200_CHECK(dense64_tree(c, dense_first));
   float ms = 0;
   cudaEventElapsedTime(&ms, c.ev[14], c.ev[15]);
   c.ms[0] = ms;
@@ -423,7 +430,7 @@ static b200fmm_status execute_body(Context &c, unsigned ops) {
     if (c.cfg.precision == B200FMM_MIXED)
       st = run_m2l_tc(c, -1);  // one launch for every level
     else
-      for (int l = 2; l <= LL && st == B200FMM_OK; ++l) st = run_m2l_fp64(c, l);
+      st = run_m2l_fp64(c, -1);
     c.mmax_ready = false;
     B200_CHECK(st);
   }

@@ -68,7 +68,7 @@ struct IListTable {
 };
 
 struct DenseTC;  // tensor-core M2L state (m2l_tc.cu)
-struct Sym64;    // two-GEMM FP64 symmetric M2L state (m2l_sym64.cu)
+struct Sym64;    // FP64 GEMM M2L state (m2l_sym64.cu)
 
 struct Context {
   b200fmm_config cfg{};
@@ -114,7 +114,8 @@ struct Context {
   long long *d_toff = nullptr;       // [343] element offset of slot t's Ut / Vt, -1 for near slots
   int *d_trank = nullptr;            // [343] rank of slot t (its class's rank)
 
-  // dense FP64 operators (CHEB_DENSE / LAGRANGE in FP64): [343][nn][nn], zero for near slots
+  // dense FP64 operators (CHEB_DENSE / LAGRANGE): [343][nn][nn rounded up to 8], zero for near slots and in the
+  // padding; kept after create() only in FP64
   double *d_dense = nullptr;
 
   IListTable itab{};
@@ -209,7 +210,7 @@ bool tc_lowrank_info(const Context &c, int *rank_of_slot, double *rank_fed);
 void slot_symmetry_tables(int p, std::vector<int> &pind, std::vector<int> &pvec);
 b200fmm_status sym_slot_factors(const Context &c, std::vector<double> &Ut, std::vector<double> &Vt,
                                 std::vector<long long> &toff, std::vector<int> &trank);
-b200fmm_status build_dense_operators(Context &c);
+b200fmm_status build_dense_operators(Context &c, int ld);  // rows of ld >= p^3 values
 // tree.cu
 b200fmm_status build_ilists(Context &c);
 b200fmm_status build_tree(Context &c, const double *x, const double *y, const double *z, const double *q,
@@ -229,13 +230,17 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard = nullptr
 // Orders the leaves by (x, y) column, z within a column (stable from Morton order), into d_leaf_rank, and
 // lays out the FP32 source records in that order (d_rec_base).  Uses the free tree-build scratch.
 b200fmm_status leaf_column_order(Context &c);
-// m2l_fp64.cu
+// m2l_fp64.cu; level < 0: every level
 b200fmm_status run_m2l_fp64(Context &c, int level);
-// m2l_sym64.cu: the FP64 symmetric M2L as two GEMMs per level (stacked V_t^T, then concatenated U_t)
+// m2l_sym64.cu: the FP64 M2L as GEMMs over one level or all (level < 0): stacked V_t^T, then the U_t or K_t
 b200fmm_status sym64_prepare(Context &c, const double *d_Ut, const double *d_Vt, const std::vector<long long> &toff,
                              const std::vector<int> &trank);
 void sym64_free(Context &c);
-b200fmm_status run_m2l_sym64(Context &c, int level);
+b200fmm_status dense64_prepare(Context &c);
+// dense operators: the tree's tables, queued (with the 344 words copied to the host) and then finished after a wait
+b200fmm_status dense64_tree_counts(Context &c, int *host_first);
+b200fmm_status dense64_tree(Context &c, const int *host_first);
+b200fmm_status run_m2l_gemm64(Context &c, int level);
 // rows of the stacked V of each source parity (the ranks of the slots that parity feeds)
 bool sym64_fed_ranks(const Context &c, double *fed);
 // m2l_tc.cu

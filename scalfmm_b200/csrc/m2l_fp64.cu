@@ -5,9 +5,8 @@
 //    16 compressed operators as Y = V^T M' then scale * U Y per class, and adds the result back through the
 //    same permutation.  Here the permutation is folded into per-slot factors U_t, V_t once (precompute.cu),
 //    and one CTA applies them for 32 targets of one child type -- which share their 189 slots -- keeping the
-//    local sums in registers.
-//  * CHEB_DENSE / LAGRANGE: L[m] += scale * sum_n K_t(X_m, Y_n) M[n] (FChebDenseKernel::M2L,
-//    FChebDenseKernel.hpp:116-127; FUnifKernel applies the same Toeplitz operator through FFTs).
+//    local sums in registers.  Kept for trees whose Y would exceed the cap of the GEMM form (m2l_sym64.cu).
+//  * CHEB_DENSE / LAGRANGE: the GEMM form.
 //  scale = 2 / cell width (FInterpMatrixKernelR::getScaleFactor, FInterpMatrixKernel.hpp:124-133).
 #include "common.cuh"
 
@@ -168,92 +167,66 @@ __global__ void __launch_bounds__(SYM_THREADS) m2l_sym_kernel(SymArgs a) {
   }
 }
 
-__global__ void m2l_dense_kernel(int p, int R, double scale, const long long *__restrict__ keys,
-                                 const int *__restrict__ ilist, const IListTable *__restrict__ itab,
-                                 const double *__restrict__ K, const double *__restrict__ M, double *__restrict__ L) {
-  extern __shared__ double sM[];
-  const int nn = p * p * p;
-  const long long c = blockIdx.x;
-  const int ct = (int)(keys[c] & 7);
-  for (int r = 0; r < R; ++r) {
-    double acc[4] = {0, 0, 0, 0};
-    for (int e = 0; e < 189; ++e) {
-      const int src = ilist[c * 189 + e];
-      if (src < 0) continue;
-      const int t = itab->slot[ct][e];
-      __syncthreads();
-      for (int i = threadIdx.x; i < nn; i += blockDim.x) sM[i] = M[((long long)src * R + r) * nn + i];
-      __syncthreads();
-      const double *Kt = K + (long long)t * nn * nn;
-      for (int k = 0; k < 4; ++k) {
-        const int m = threadIdx.x + k * blockDim.x;
-        if (m >= nn) break;
-        double s = 0.0;
-        for (int n = 0; n < nn; ++n) s += Kt[(long long)n * nn + m] * sM[n];
-        acc[k] += s;
-      }
-    }
-    for (int k = 0; k < 4; ++k) {
-      const int m = threadIdx.x + k * blockDim.x;
-      if (m < nn) L[(c * R + r) * nn + m] += scale * acc[k];
-    }
-  }
-}
-
 }  // namespace
 
-b200fmm_status run_m2l_fp64(Context &c, int level) {
-  if (level < 2 || level > c.H - 1) return fail(B200FMM_ERR_INVALID, "m2l: level must be in [2, height-1]");
+// CHEB_SYM by the per-target kernel, one level.
+static b200fmm_status run_m2l_sym(Context &c, int level) {
   const Level &T = c.lv[level];
   if (T.n == 0) return B200FMM_OK;
-  const double scale = 2.0 / (c.cfg.box_width / (double)(1LL << level));
-  if (c.cfg.kernel == B200FMM_CHEB_SYM && c.cfg.precision == B200FMM_FP64) {
-    // the two-GEMM form (m2l_sym64.cu); the per-target kernel below remains for trees whose largest level
-    // would need more than the two-GEMM form's cap on Y, and on request (B200FMM_SYM64=0)
-    const char *env = std::getenv("B200FMM_SYM64");
-    if (c.s64 && !(env && env[0] == '0')) {
-      const b200fmm_status st = run_m2l_sym64(c, level);
-      if (st != B200FMM_ERR_UNSUPPORTED) return st;
-    }
-    SymArgs a;
-    a.R = c.R;
-    a.scale = scale;
-    a.nparents = c.lv[level - 1].n;
-    a.child = c.lv[level - 1].child;
-    a.ilist = T.ilist;
-    a.itab = c.d_itab;
-    a.Ut = c.d_Ut;
-    a.Vt = c.d_Vt;
-    a.toff = c.d_toff;
-    a.trank = c.d_trank;
-    a.M = T.M;
-    a.L = T.L;
-    a.max_rank = c.max_rank;
-    const int T = SYM_T;
-    const size_t sh = sizeof(double) * ((size_t)T * c.nn + (size_t)T * c.max_rank + (size_t)c.nn * c.max_rank);
-    if (sh > 227 * 1024) return fail(B200FMM_ERR_UNSUPPORTED, "compressed operators too large for the FP64 M2L kernel");
-    const dim3 grid((unsigned)((a.nparents + T - 1) / T), 8);
-    for (int r = 0; r < c.R; ++r) {
-      a.rhs = r;
-      switch (c.p) {
+  SymArgs a;
+  a.R = c.R;
+  a.scale = 2.0 / (c.cfg.box_width / (double)(1LL << level));
+  a.nparents = c.lv[level - 1].n;
+  a.child = c.lv[level - 1].child;
+  a.ilist = T.ilist;
+  a.itab = c.d_itab;
+  a.Ut = c.d_Ut;
+  a.Vt = c.d_Vt;
+  a.toff = c.d_toff;
+  a.trank = c.d_trank;
+  a.M = T.M;
+  a.L = T.L;
+  a.max_rank = c.max_rank;
+  const int ST = SYM_T;
+  const size_t sh = sizeof(double) * ((size_t)ST * c.nn + (size_t)ST * c.max_rank + (size_t)c.nn * c.max_rank);
+  if (sh > 227 * 1024) return fail(B200FMM_ERR_UNSUPPORTED, "compressed operators too large for the FP64 M2L kernel");
+  const dim3 grid((unsigned)((a.nparents + ST - 1) / ST), 8);
+  for (int r = 0; r < c.R; ++r) {
+    a.rhs = r;
+    switch (c.p) {
 #define B200_SYM(PV)                                                                                        \
   case PV:                                                                                                  \
     B200_CUDA(cudaFuncSetAttribute(m2l_sym_kernel<PV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh)); \
     m2l_sym_kernel<PV><<<grid, SYM_THREADS, sh, c.stream>>>(a);                                             \
     break;
-        B200_SYM(3) B200_SYM(4) B200_SYM(5) B200_SYM(6) B200_SYM(7) B200_SYM(8)
+      B200_SYM(3) B200_SYM(4) B200_SYM(5) B200_SYM(6) B200_SYM(7) B200_SYM(8)
 #undef B200_SYM
-        default:
-          return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
-      }
-      ++c.launches;
+      default:
+        return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
     }
-  } else {
-    m2l_dense_kernel<<<(unsigned)T.n, 128, sizeof(double) * c.nn, c.stream>>>(
-        c.p, c.R, scale, T.keys, T.ilist, c.d_itab, c.d_dense, T.M, T.L);
     ++c.launches;
   }
   B200_CUDA(cudaGetLastError());
+  return B200FMM_OK;
+}
+
+// level < 0: every level
+b200fmm_status run_m2l_fp64(Context &c, int level) {
+  if (level > c.H - 1 || level == 0 || level == 1)
+    return fail(B200FMM_ERR_INVALID, "m2l: level must be in [2, height-1]");
+  // the GEMM form (m2l_sym64.cu); for CHEB_SYM the per-target kernel above remains for levels whose Y would
+  // exceed the GEMM form's cap, and on request (B200FMM_SYM64=0)
+  const bool sym = c.cfg.kernel == B200FMM_CHEB_SYM;
+  const char *env = std::getenv("B200FMM_SYM64");
+  if (!sym || !(env && env[0] == '0')) {
+    const b200fmm_status st = run_m2l_gemm64(c, level);
+    if (!sym || st != B200FMM_ERR_UNSUPPORTED) return st;
+    if (level < 0) {
+      for (int l = 2; l < c.H; ++l) B200_CHECK(run_m2l_fp64(c, l));
+      return B200FMM_OK;
+    }
+  }
+  for (int l = level < 0 ? 2 : level; l <= (level < 0 ? c.H - 1 : level); ++l) B200_CHECK(run_m2l_sym(c, l));
   return B200FMM_OK;
 }
 

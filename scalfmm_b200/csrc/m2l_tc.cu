@@ -2299,7 +2299,7 @@ b200fmm_status tc_init(Context &c) {
   t->ncols = 32;
   while (t->ncols < t->nbuf * t->NP) t->ncols *= 2;
   if (!lr) {
-    B200_CHECK(build_dense_operators(c));  // FP64 K on the device
+    B200_CHECK(build_dense_operators(c, nn));  // FP64 K on the device
     const size_t bsz = (size_t)343 * t->NP * t->KP;
     B200_CUDA(cudaMalloc(&t->Bhi, bsz * sizeof(__half)));
     B200_CUDA(cudaMalloc(&t->Blo, bsz * sizeof(__half)));

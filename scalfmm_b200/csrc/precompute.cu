@@ -126,22 +126,23 @@ __global__ void eval_weighted_classes(int p, const double *__restrict__ roots, c
   A[(long long)c * nn * nn + e] = w[t] * w[s] * (1.0 / sqrt(dx * dx + dy * dy + dz * dz));
 }
 
-// Dense operators for every far slot: K[t][n][m] = 1/|X_m - Y_n| (zero for the 27 near slots).
-__global__ void eval_dense(int p, const double *__restrict__ roots, double *__restrict__ K) {
+// Dense operators for every far slot: K[t][n][m] = 1/|X_m - Y_n| (zero for the 27 near slots and for the padding
+// p^3 <= m < ld).
+__global__ void eval_dense(int p, int ld, const double *__restrict__ roots, double *__restrict__ K) {
   const int nn = p * p * p;
   const int t = blockIdx.y;
   const int i = t / 49 - 3, j = (t / 7) % 7 - 3, k = t % 7 - 3;
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= (long long)nn * nn) return;
+  if (e >= (long long)nn * ld) return;
   double v = 0.0;
-  if (abs(i) > 1 || abs(j) > 1 || abs(k) > 1) {
-    const int n = (int)(e / nn), m = (int)(e % nn);  // stored [t][n][m]: coalesced over the target node m
+  const int n = (int)(e / ld), m = (int)(e % ld);  // stored [t][n][m]: coalesced over the target node m
+  if (m < nn && (abs(i) > 1 || abs(j) > 1 || abs(k) > 1)) {
     const double dx = roots[m % p] - (2.0 * i + roots[n % p]);
     const double dy = roots[(m / p) % p] - (2.0 * j + roots[(n / p) % p]);
     const double dz = roots[m / (p * p)] - (2.0 * k + roots[n / (p * p)]);
     v = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
   }
-  K[(long long)t * nn * nn + e] = v;
+  K[(long long)t * nn * ld + e] = v;
 }
 
 }  // namespace
@@ -364,11 +365,11 @@ b200fmm_status upload_sym_operators(Context &c) {
   return B200FMM_OK;
 }
 
-b200fmm_status build_dense_operators(Context &c) {
+b200fmm_status build_dense_operators(Context &c, int ld) {
   const int nn = c.nn;
   if (c.d_dense) return B200FMM_OK;
-  B200_CUDA(cudaMalloc(&c.d_dense, sizeof(double) * 343 * (size_t)nn * nn));
-  eval_dense<<<dim3(grid_for((long long)nn * nn, 256), 343), 256>>>(c.p, c.d_roots, c.d_dense);
+  B200_CUDA(cudaMalloc(&c.d_dense, sizeof(double) * 343 * (size_t)nn * ld));
+  eval_dense<<<dim3(grid_for((long long)nn * ld, 256), 343), 256>>>(c.p, ld, c.d_roots, c.d_dense);
   B200_CUDA(cudaGetLastError());
   B200_CUDA(cudaDeviceSynchronize());
   return B200FMM_OK;

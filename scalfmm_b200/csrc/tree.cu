@@ -687,7 +687,7 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
   cudaStream_t s = c.stream;
   c.tree_launches = 0;
   c.packed32 = false;
-  if (!c.h_pinned) B200_CUDA(cudaMallocHost((void **)&c.h_pinned, sizeof(long long) * 64));
+  if (!c.h_pinned) B200_CUDA(cudaMallocHost((void **)&c.h_pinned, sizeof(long long) * 64 + sizeof(int) * 344));
   // particle-sized buffers
   size_t cap;
   cap = c.cap_N;

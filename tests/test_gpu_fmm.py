@@ -196,6 +196,43 @@ def test_operation_masks_match_oracle(golden, ops):
             assert S.rel_l2(r[f], o[f]) < 1e-12, f
 
 
+@pytest.mark.parametrize("kernel,order,height,n,dist,nrhs", [
+    # sizes around the 64-cell tiles and the row tiles of every order, K tails of p^3 mod 4, split and unsplit K
+    ("cheb_sym", 3, 4, 700, "plummer", 1), ("cheb_sym", 4, 5, 1500, "ellipsoid", 3), ("cheb_sym", 5, 5, 9000, "uniform", 1),
+    ("cheb_sym", 6, 4, 3000, "uniform", 2), ("cheb_sym", 7, 4, 900, "plummer", 1), ("cheb_sym", 8, 4, 500, "ellipsoid", 1),
+    ("cheb_sym", 8, 3, 20, "uniform", 1), ("cheb_dense", 3, 5, 3000, "uniform", 2), ("cheb_dense", 4, 4, 1000, "plummer", 1),
+    ("cheb_dense", 5, 4, 1500, "uniform", 3), ("cheb_dense", 7, 4, 500, "ellipsoid", 1), ("cheb_dense", 8, 3, 60, "plummer", 1),
+    ("lagrange", 6, 5, 2500, "ellipsoid", 2), ("lagrange", 7, 3, 300, "uniform", 1), ("lagrange", 5, 3, 2, "uniform", 1),
+])
+def test_fp64_gemm_m2l_matches_oracle(kernel, order, height, n, dist, nrhs):
+    from distributions import ellipsoid_surface, plummer
+
+    rng = np.random.default_rng(order * 100 + n)
+    x, y, z = {"uniform": lambda: rng.random((3, n)), "plummer": lambda: plummer(n, 7),
+               "ellipsoid": lambda: ellipsoid_surface(n, 7)}[dist]()
+    q = rng.uniform(-1, 1, (nrhs, n) if nrhs > 1 else n)
+    f = S.FMM(kernel, order, height, nrhs=nrhs)
+    sym = dict(zip(("sym_ranks", "sym_uv"), f.get_sym_operators())) if kernel == "cheb_sym" else {}
+    f.set_particles(x, y, z, q.ravel())
+    f.execute()
+    whole = f.results()
+    o = O.fmm(S.KERNELS[kernel], order, height, 1.0, CENTER, x, y, z, q, **sym)
+    # the far field level by level, in the form that a single level takes
+    f.reset_expansions()
+    f.execute(S.ALL & ~(S.M2L | S.L2L | S.L2P | S.P2P))
+    for lvl in range(2, height):
+        f.m2l(lvl)
+    for lvl in range(2, height - 1):
+        f.l2l(lvl)
+    f.l2p()
+    f.p2p(0)
+    single = f.results()
+    f.close()
+    for k in FIELDS:
+        assert S.rel_l2(whole[k], o[k]) < 1e-12, (k, S.rel_l2(whole[k], o[k]))
+        assert S.rel_l2(single[k], o[k]) < 1e-12, (k, S.rel_l2(single[k], o[k]))
+
+
 def test_level_batched_operators_equal_execute(golden):
     g = golden("fmm_sym_p4_h5_n3000.npz")
     sym = golden("sym_ops_p4.npz")
