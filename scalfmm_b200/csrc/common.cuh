@@ -230,6 +230,8 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard = nullptr
 // Orders the leaves by (x, y) column, z within a column (stable from Morton order), into d_leaf_rank, and
 // lays out the FP32 source records in that order (d_rec_base).  Uses the free tree-build scratch.
 b200fmm_status leaf_column_order(Context &c);
+// d_chunk_base: the near field's work items, leaf by leaf (p2p_leaf_items).  Uses the same scratch.
+b200fmm_status leaf_items(Context &c, int whole, int item);
 // m2l_fp64.cu; level < 0: every level
 b200fmm_status run_m2l_fp64(Context &c, int level);
 // m2l_sym64.cu: the FP64 M2L as GEMMs over one level or all (level < 0): stacked V_t^T, then the U_t or K_t

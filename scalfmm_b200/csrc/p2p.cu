@@ -5,8 +5,8 @@
 // The reference evaluates each unordered pair once (mutual half shell, FChebSymKernel.hpp:468-478);
 // the ordered pairs summed here per target are the same set.
 //
-//  * FP64 (parity form): one CTA per target leaf, source leaves staged through shared memory, the
-//    reference's arithmetic sequence (1/r^2, sqrt, products).
+//  * FP64 (parity form): one CTA per 32 targets of a leaf, the sources of the leaf and its neighbours staged through
+//    shared memory, rsqrt() in FP64.
 //  * FP32 (mixed form), two source particles per step with Blackwell's packed FP32x2 instructions
 //    (add/mul/fma.f32x2): positions relative to the box corner as a float pair (hi, lo), so that per pair
 //    dx = (t_hi - s_hi) + (t_lo - s_lo) with the first difference exact for nearby particles (Sterbenz),
@@ -23,66 +23,151 @@ namespace b200 {
 
 namespace {
 
-constexpr int P2P64_THREADS = 64;
+constexpr int P2P64_WARPS = 4, P2P64_THREADS = 32 * P2P64_WARPS;
+constexpr int P2P64_TGT = 32;  // targets per work item
 
-// shard (optional): [first leaf, end leaf) of the targets to evaluate
-__global__ void p2p_fp64_kernel(int R, long long N, const long long *__restrict__ leaf_start,
-                                const int *__restrict__ nbr, int variant, const double *__restrict__ x,
-                                const double *__restrict__ y, const double *__restrict__ z,
-                                const double *__restrict__ q, double *__restrict__ phi, double *__restrict__ fx,
-                                double *__restrict__ fy, double *__restrict__ fz, const long long *__restrict__ shard) {
-  __shared__ double sx[P2P64_THREADS], sy[P2P64_THREADS], sz[P2P64_THREADS], sq[P2P64_THREADS];
-  __shared__ long long sidx[P2P64_THREADS];
-  const long long leaf = blockIdx.x;
-  if (shard && (leaf < shard[0] || leaf >= shard[1])) return;
-  const long long t0 = leaf_start[leaf], t1 = leaf_start[leaf + 1];
-  for (int r = 0; r < R; ++r) {
-    const double *qr = q + (long long)r * N;
-    for (long long tb = t0; tb < t1; tb += blockDim.x) {
-      const long long i = tb + threadIdx.x;
-      const bool active = i < t1;
-      const double tx = active ? x[i] : 0, ty = active ? y[i] : 0, tz = active ? z[i] : 0;
-      const double tq = active ? qr[i] : 0;
-      double pv = 0, gx = 0, gy = 0, gz = 0;
-      for (int e = 0; e < 27; ++e) {
-        if (variant == 1 && e == 13) continue;
-        const int sl = nbr[leaf * 27 + e];
-        if (sl < 0) continue;
-        const long long s0 = leaf_start[sl], s1 = leaf_start[sl + 1];
-        for (long long sb = s0; sb < s1; sb += blockDim.x) {
-          __syncthreads();
-          const long long j = sb + threadIdx.x;
-          if (j < s1) {
-            sx[threadIdx.x] = x[j];
-            sy[threadIdx.x] = y[j];
-            sz[threadIdx.x] = z[j];
-            sq[threadIdx.x] = qr[j];
-            sidx[threadIdx.x] = j;
-          }
-          __syncthreads();
-          const int cnt = (int)min((long long)blockDim.x, s1 - sb);
-          if (active) {
-            for (int k = 0; k < cnt; ++k) {
-              if (sidx[k] == i) continue;
-              double dx = tx - sx[k], dy = ty - sy[k], dz = tz - sz[k];
-              double inv2 = 1.0 / (dx * dx + dy * dy + dz * dz);
-              const double inv = sqrt(inv2);
-              inv2 *= inv;
-              inv2 *= tq * sq[k];
-              gx += -dx * inv2;
-              gy += -dy * inv2;
-              gz += -dz * inv2;
-              pv += inv * sq[k];
-            }
-          }
+// The pairs of NR right-hand sides of one source with one target; SELF: the source may be the target itself.
+template <int NR, bool SELF>
+__device__ __forceinline__ void p2p64_pair(const double4 &s, bool self, const double *__restrict__ sq, int sq_stride,
+                                           double tx, double ty, double tz, double (&pv)[NR], double (&gx)[NR],
+                                           double (&gy)[NR], double (&gz)[NR]) {
+  const double dx = tx - s.x, dy = ty - s.y, dz = tz - s.z;
+  double inv = rsqrt(dx * dx + dy * dy + dz * dz);
+  if (SELF && self) inv = 0.0;
+  const double inv2 = inv * inv;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const double p = inv * (NR == 1 ? s.w : sq[r * sq_stride]);
+    const double f = p * inv2;
+    pv[r] += p;
+    gx[r] += dx * f;
+    gy[r] += dy * f;
+    gz[r] += dz * f;
+  }
+}
+
+// FP64.  One CTA per work item (up to 32 targets of a leaf, c.d_chunk_base); the sources of the leaf and its
+// neighbours are one sequence, staged 128 at a time, and each warp takes 32 of them against all the item's targets
+// (lane = target; 16 or 8 targets are replicated over 2 or 4 lane groups with every 2nd or 4th source).  The warps'
+// sums are added at the end in a fixed order.  What bounds it is the FP64 pipe: per pair 3 differences, 3 for r^2,
+// the reciprocal square root (about 9 instructions of rsqrt(); the division and square root of sqrt(1 / r^2) that
+// the reference writes take about 22) and 7 for the sums: 1M uniform points in leaves of 30: 3.85 -> 1.53 ms (0.51
+// Tpairs/s), 500,009 on a surface 2.05 -> 0.82 ms; 60,000 clustered points, whose dense leaves one CTA each carried
+// before, 9.1 -> 0.39 ms.  Against sums in extended precision the error is 0.3-0.6 of the earlier kernel's (shorter
+// chains of additions).  shard (optional): [first leaf, end leaf) of the targets.
+template <int NR>
+__global__ void __launch_bounds__(P2P64_THREADS) p2p_fp64_kernel(
+    int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
+    const long long *__restrict__ chunk_base, int variant, const double *__restrict__ x, const double *__restrict__ y,
+    const double *__restrict__ z, const double *__restrict__ q, double *__restrict__ phi, double *__restrict__ fx,
+    double *__restrict__ fy, double *__restrict__ fz, const long long *__restrict__ shard) {
+  __shared__ __align__(32) double4 src[P2P64_THREADS];              // x, y, z, q (of the only right-hand side)
+  __shared__ double srcq[NR > 1 ? NR : 1][NR > 1 ? P2P64_THREADS : 1];
+  __shared__ double red[P2P64_WARPS - 1][4][32];
+  __shared__ long long s_first[27];   // first particle of each neighbour present
+  __shared__ int s_off[28], s_n, s_self;  // where its sources begin in the sequence; which one is the leaf itself
+  const long long leaf_lo = shard ? shard[0] : 0, leaf_hi = shard ? shard[1] : nleaves;
+  const long long item = chunk_base[leaf_lo] + blockIdx.x;
+  if (item >= chunk_base[leaf_hi]) return;
+  long long leaf = leaf_lo, hi = leaf_hi - 1;  // the last leaf whose first item is <= item
+  while (leaf < hi) {
+    const long long mid = (leaf + hi + 1) >> 1;
+    if (chunk_base[mid] <= item)
+      leaf = mid;
+    else
+      hi = mid - 1;
+  }
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  if (w == 0) {
+    int nb = lane < 27 ? nbr[leaf * 27 + lane] : -1;
+    if (variant == 1 && lane == 13) nb = -1;
+    const long long a = nb >= 0 ? leaf_start[nb] : 0;
+    const int cnt = nb >= 0 ? (int)(leaf_start[nb + 1] - a) : 0;
+    int e = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, e, o);
+      if (lane >= o) e += v;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, cnt > 0);
+    const int k = __popc(m & ((1u << lane) - 1u));
+    if (cnt > 0) {
+      s_first[k] = a;
+      s_off[k] = e - cnt;
+    }
+    if (lane == 13) s_self = cnt > 0 ? k : -1;
+    if (lane == 31) {
+      s_n = __popc(m);
+      s_off[__popc(m)] = e;
+    }
+  }
+  __syncthreads();
+  const int nn = s_n, total = s_off[nn], self = s_self;
+  const long long t0 = leaf_start[leaf] + P2P64_TGT * (item - chunk_base[leaf]);
+  const int m = (int)min((long long)P2P64_TGT, leaf_start[leaf + 1] - t0);
+  const int T = m <= 8 ? 8 : (m <= 16 ? 16 : 32), G = 32 / T;
+  const int tl = lane & (T - 1), g = lane / T;
+  const bool active = tl < m;
+  const double tx = active ? x[t0 + tl] : 0, ty = active ? y[t0 + tl] : 0, tz = active ? z[t0 + tl] : 0;
+  // the sequence position of the target itself
+  const int own = self >= 0 ? s_off[self] + (int)(t0 - s_first[self]) + tl : -1;
+  const int own0 = self >= 0 ? s_off[self] : -1, own1 = self >= 0 ? s_off[self + 1] : -1;
+  for (int r0 = 0; r0 < R; r0 += NR) {
+    double pv[NR], gx[NR], gy[NR], gz[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) pv[r] = gx[r] = gy[r] = gz[r] = 0.0;
+    for (int sb = 0; sb < total; sb += P2P64_THREADS) {
+      __syncthreads();
+      const int k = sb + t;
+      if (k < total) {
+        int a = 0, b = nn - 1;  // the last neighbour that begins at or before k
+        while (a < b) {
+          const int mid = (a + b + 1) >> 1;
+          if (s_off[mid] <= k)
+            a = mid;
+          else
+            b = mid - 1;
         }
+        const long long j = s_first[a] + (k - s_off[a]);
+        src[t] = make_double4(x[j], y[j], z[j], NR == 1 ? q[(long long)r0 * N + j] : 0.0);
+        if (NR > 1)
+#pragma unroll
+          for (int r = 0; r < NR; ++r) srcq[r][t] = r0 + r < R ? q[(long long)(r0 + r) * N + j] : 0.0;
       }
-      if (active) {
-        const long long j = (long long)r * N + i;
-        phi[j] += pv;
-        fx[j] += gx;
-        fy[j] += gy;
-        fz[j] += gz;
+      __syncthreads();
+      const int i1 = min(32 * w + 32, total - sb);
+      if (sb + i1 > own0 && sb + 32 * w < own1) {
+        for (int i = 32 * w + g; i < i1; i += G)
+          p2p64_pair<NR, true>(src[i], sb + i == own, &srcq[0][i], P2P64_THREADS, tx, ty, tz, pv, gx, gy, gz);
+      } else {
+#pragma unroll 4
+        for (int i = 32 * w + g; i < i1; i += G)
+          p2p64_pair<NR, false>(src[i], false, &srcq[0][i], P2P64_THREADS, tx, ty, tz, pv, gx, gy, gz);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      if (r0 + r >= R) break;
+      double v[4] = {pv[r], gx[r], gy[r], gz[r]};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        for (int o = T; o < 32; o <<= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+      __syncthreads();
+      if (w > 0)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) red[w - 1][c][lane] = v[c];
+      __syncthreads();
+      if (w == 0 && active && g == 0) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int u = 0; u < P2P64_WARPS - 1; ++u) v[c] += red[u][c][lane];
+        const long long j = (long long)(r0 + r) * N + t0 + tl;
+        const double nq = -q[j];
+        phi[j] += v[0];
+        fx[j] += nq * v[1];
+        fy[j] += nq * v[2];
+        fz[j] += nq * v[3];
       }
     }
   }
@@ -788,10 +873,16 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     B200_CUDA(record_event(c, 11));
     ++c.launches;
   } else {
+    if (c.column_serial != c.tree_serial) {
+      B200_CHECK(leaf_items(c, P2P64_TGT, P2P64_TGT));
+      c.column_serial = c.tree_serial;
+    }
     B200_CUDA(record_event(c, 10));
-    p2p_fp64_kernel<<<(unsigned)L.n, P2P64_THREADS, 0, c.stream>>>(c.R, c.N, c.d_leaf_start, c.d_leaf_nbr, variant,
-                                                                   c.d_x, c.d_y, c.d_z, c.d_q, c.d_phi, c.d_fx,
-                                                                   c.d_fy, c.d_fz, shard);
+    // nleaves + N / 32 bounds the work items; several right-hand sides share a pair's geometry four at a time
+    const unsigned blocks = grid_for(L.n + c.N / P2P64_TGT, 1);
+    auto kernel = c.R > 1 ? p2p_fp64_kernel<4> : p2p_fp64_kernel<1>;
+    kernel<<<blocks, P2P64_THREADS, 0, c.stream>>>(c.R, c.N, L.n, c.d_leaf_start, c.d_leaf_nbr, c.d_chunk_base, variant,
+                                                   c.d_x, c.d_y, c.d_z, c.d_q, c.d_phi, c.d_fx, c.d_fy, c.d_fz, shard);
     B200_CUDA(record_event(c, 11));
     ++c.launches;
   }

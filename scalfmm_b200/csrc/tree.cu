@@ -962,11 +962,17 @@ b200fmm_status leaf_column_order(Context &c) {
   leaf_rank_kernel<<<grid_for(nl, 256), 256, 0, s>>>(nl, v0, c.d_leaf_start, c.d_leaf_rank, nrec);
   B200_CHECK(scan_i64(c, nrec, c.d_rec_base, nl, (long long *)c.d_scan));
   rec_total_kernel<<<1, 1, 0, s>>>(nl, nrec, c.d_rec_base);
-  // the near field's work items, leaf by leaf (nrec is free again)
-  leaf_chunks_kernel<<<grid_for(nl, 256), 256, 0, s>>>(nl, c.d_leaf_start, c.p2p_whole, c.p2p_item, nrec);
-  B200_CHECK(scan_i64(c, nrec, c.d_chunk_base, nl, (long long *)c.d_scan));
-  rec_total_kernel<<<1, 1, 0, s>>>(nl, nrec, c.d_chunk_base);
-  c.launches += 4;
+  c.launches += 2;
+  return leaf_items(c, c.p2p_whole, c.p2p_item);
+}
+
+b200fmm_status leaf_items(Context &c, int whole, int item) {
+  const long long nl = c.lv[c.H - 1].n;
+  long long *nch = c.d_flags;
+  leaf_chunks_kernel<<<grid_for(nl, 256), 256, 0, c.stream>>>(nl, c.d_leaf_start, whole, item, nch);
+  B200_CHECK(scan_i64(c, nch, c.d_chunk_base, nl, (long long *)c.d_scan));
+  rec_total_kernel<<<1, 1, 0, c.stream>>>(nl, nch, c.d_chunk_base);
+  c.launches += 2;
   B200_CUDA(cudaGetLastError());
   return B200FMM_OK;
 }

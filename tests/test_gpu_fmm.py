@@ -196,6 +196,41 @@ def test_operation_masks_match_oracle(golden, ops):
             assert S.rel_l2(r[f], o[f]) < 1e-12, f
 
 
+@pytest.mark.parametrize("precision,nrhs", [("fp64", 1), ("fp64", 3), ("fp64", 5), ("mixed", 1), ("mixed", 3)])
+@pytest.mark.parametrize("variant", [0, 1])
+def test_near_field_over_leaf_sizes(precision, nrhs, variant):
+    """Leaves at the edges of the kernels' target chunks (8, 16, 32, 48, 64), source stages and work items, a leaf far
+    larger than the rest and an isolated one, against a sum in NumPy."""
+    rng = np.random.default_rng(11)
+    counts = [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 96, 97, 129, 700]
+    side = 8
+    leaves = [(x, y, z) for x in range(3) for y in range(3) for z in range(3)][:len(counts)] + [(7, 7, 7)]
+    pos = np.concatenate([(np.array(c)[:, None] + rng.uniform(0.02, 0.98, (3, k))) / side
+                          for c, k in zip(leaves, counts + [5])], axis=1)
+    pos = pos[:, rng.permutation(pos.shape[1])].copy()
+    n = pos.shape[1]
+    q = rng.uniform(-1, 1, (nrhs, n))
+    f = S.FMM("cheb_dense", 3, 4, nrhs=nrhs, precision=precision)
+    f.set_particles(pos[0], pos[1], pos[2], q.ravel())
+    f.zero_results()
+    f.p2p(variant)
+    r = f.results()
+    f.close()
+    cell = np.floor(pos * side).astype(int)
+    gap = np.abs(cell[:, :, None] - cell[:, None, :]).max(axis=0)
+    d = pos[:, :, None] - pos[:, None, :]
+    with np.errstate(divide="ignore"):
+        inv = 1.0 / np.sqrt((d * d).sum(axis=0))
+    inv[(gap > 1) | (gap < variant) | np.eye(n, dtype=bool)] = 0.0
+    # FP64: a few roundings of 1.1e-16 per pair and sums of ~1,000 terms; MIXED: about six FP32 roundings (6e-8) per
+    # pair, positions to 48 bits, compensated sums
+    tol = 1e-13 if precision == "fp64" else 5e-7
+    for k in range(nrhs):
+        assert S.rel_l2(r["phi"].reshape(nrhs, n)[k], inv @ q[k]) < tol
+        for a, name in enumerate(("fx", "fy", "fz")):
+            assert S.rel_l2(r[name].reshape(nrhs, n)[k], -q[k] * ((d[a] * inv ** 3) @ q[k])) < tol
+
+
 @pytest.mark.parametrize("kernel,order,height,n,dist,nrhs", [
     # sizes around the 64-cell tiles and the row tiles of every order, K tails of p^3 mod 4, split and unsplit K
     ("cheb_sym", 3, 4, 700, "plummer", 1), ("cheb_sym", 4, 5, 1500, "ellipsoid", 3), ("cheb_sym", 5, 5, 9000, "uniform", 1),
