@@ -7,13 +7,13 @@
 //
 //  * FP64 (parity form): one CTA per 32 targets of a leaf, the sources of the leaf and its neighbours staged through
 //    shared memory, rsqrt() in FP64.
-//  * FP32 (mixed form), two source particles per step with Blackwell's packed FP32x2 instructions
-//    (add/mul/fma.f32x2): positions relative to the box corner as a float pair (hi, lo), so that per pair
+//  * FP32 (mixed form), two source particles against two targets per lane and step with Blackwell's packed FP32x2
+//    instructions (add/mul/fma.f32x2): positions relative to the box corner as a float pair (hi, lo), so that per pair
 //    dx = (t_hi - s_hi) + (t_lo - s_lo) with the first difference exact for nearby particles (Sterbenz),
 //    which keeps the close pairs -- the ones that dominate the forces -- accurate to a few ulp.  One warp per
-//    target leaf; the neighbour leaves are walked as contiguous runs of records (one per neighbour column)
+//    leaf or piece of a larger one; the neighbour leaves are walked as contiguous runs of records (one per neighbour column)
 //    copied into shared memory by the bulk-copy engine (cp.async.bulk + mbarrier, 3-deep ring); rsqrt on the
-//    SFU; per-target compensated (two-sum) accumulation of the per-stage partial sums; the result is added
+//    SFU; per-target compensated (two-sum) accumulation of partial sums; the result is added
 //    in FP64 to the far field.
 #include "common.cuh"
 
@@ -244,6 +244,16 @@ __global__ void pack_records32(long long N, int R, const long long *__restrict__
   }
 }
 
+// The same for two values at once, packed.
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ void two_sum2(float2 &hi, float2 &lo, float2 v) {
+  const float2 s = __fadd2_rn(hi, v);
+  const float2 bp = __fadd2_rn(s, neg2(hi));
+  const float2 err = __fadd2_rn(__fadd2_rn(hi, neg2(__fadd2_rn(s, neg2(bp)))), __fadd2_rn(v, neg2(bp)));
+  hi = s;
+  lo = __fadd2_rn(lo, err);
+}
+
 __device__ __forceinline__ void two_sum(float &hi, float &lo, float v) {
   const float s = hi + v;
   const float bp = s - hi;
@@ -253,7 +263,9 @@ __device__ __forceinline__ void two_sum(float &hi, float &lo, float v) {
 }
 
 constexpr int P2P32_WARPS = 4;   // target leaves per CTA (one warp each)
-constexpr int P2P32_STAGE = 32;  // source records (64 particles) per bulk-copy stage: 24 KB per CTA, 7 CTAs per SM
+constexpr int P2P32_STAGE = 56;  // source records (112 particles) per bulk-copy stage
+constexpr int P2P32_FLUSH = 24;  // records per lane whose sums enter the compensated sums together
+constexpr int P2P32_TGT = 2;     // targets per lane
 constexpr int P2P32_NBUF = 3;    // stages in flight per warp
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -299,35 +311,53 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
-// One record (two sources) against the lane's target: packed FP32x2 difference, r^2, rsqrt on the SFU.
+// A lane's target: its position, each coordinate twice for the packed instructions.
+struct Target32 {
+  float2 hx, hy, hz, lx, ly, lz;
+};
+struct Sums32 {
+  float2 pv, ax, ay, az;
+};
+
+// One record (two sources) against each of the lane's targets: packed FP32x2 difference, r^2, rsqrt on the SFU.
 template <bool SELF>
-__device__ __forceinline__ void p2p_record(const float4 *__restrict__ s, int k, int self_rel, float2 th_x,
-                                           float2 th_y, float2 th_z, float2 tl_x, float2 tl_y, float2 tl_z,
-                                           float2 &pv, float2 &ax, float2 &ay, float2 &az) {
+__device__ __forceinline__ void p2p_record(const float4 *__restrict__ s, int k, const int (&self_rel)[P2P32_TGT],
+                                           const Target32 (&t)[P2P32_TGT], Sums32 (&acc)[P2P32_TGT]) {
   const float4 A = s[4 * k], B = s[4 * k + 1], C = s[4 * k + 2], D = s[4 * k + 3];
-  const float2 dx = __fadd2_rn(__fadd2_rn(th_x, make_float2(A.x, A.y)), __fadd2_rn(tl_x, make_float2(C.x, C.y)));
-  const float2 dy = __fadd2_rn(__fadd2_rn(th_y, make_float2(A.z, A.w)), __fadd2_rn(tl_y, make_float2(C.z, C.w)));
-  const float2 dz = __fadd2_rn(__fadd2_rn(th_z, make_float2(B.x, B.y)), __fadd2_rn(tl_z, make_float2(D.x, D.y)));
-  float2 r2 = __fmul2_rn(dx, dx);
-  r2 = __ffma2_rn(dy, dy, r2);
-  r2 = __ffma2_rn(dz, dz, r2);
-  float2 inv;
-  if (SELF) {
-    inv = make_float2(2 * k == self_rel ? 0.f : rsqrt_ftz(r2.x), 2 * k + 1 == self_rel ? 0.f : rsqrt_ftz(r2.y));
-  } else {
-    inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+#pragma unroll
+  for (int u = 0; u < P2P32_TGT; ++u) {
+    const float2 dx = __fadd2_rn(__fadd2_rn(t[u].hx, make_float2(A.x, A.y)), __fadd2_rn(t[u].lx, make_float2(C.x, C.y)));
+    const float2 dy = __fadd2_rn(__fadd2_rn(t[u].hy, make_float2(A.z, A.w)), __fadd2_rn(t[u].ly, make_float2(C.z, C.w)));
+    const float2 dz = __fadd2_rn(__fadd2_rn(t[u].hz, make_float2(B.x, B.y)), __fadd2_rn(t[u].lz, make_float2(D.x, D.y)));
+    float2 r2 = __fmul2_rn(dx, dx);
+    r2 = __ffma2_rn(dy, dy, r2);
+    r2 = __ffma2_rn(dz, dz, r2);
+    float2 inv;
+    if (SELF) {
+      inv = make_float2(2 * k == self_rel[u] ? 0.f : rsqrt_ftz(r2.x), 2 * k + 1 == self_rel[u] ? 0.f : rsqrt_ftz(r2.y));
+    } else {
+      inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+    }
+    const float2 qi = __fmul2_rn(make_float2(B.z, B.w), inv);
+    const float2 qi3 = __fmul2_rn(qi, __fmul2_rn(inv, inv));
+    acc[u].pv = __fadd2_rn(acc[u].pv, qi);
+    acc[u].ax = __ffma2_rn(dx, qi3, acc[u].ax);
+    acc[u].ay = __ffma2_rn(dy, qi3, acc[u].ay);
+    acc[u].az = __ffma2_rn(dz, qi3, acc[u].az);
   }
-  const float2 qi = __fmul2_rn(make_float2(B.z, B.w), inv);
-  const float2 qi3 = __fmul2_rn(qi, __fmul2_rn(inv, inv));
-  pv = __fadd2_rn(pv, qi);
-  ax = __ffma2_rn(dx, qi3, ax);
-  ay = __ffma2_rn(dy, qi3, ay);
-  az = __ffma2_rn(dz, qi3, az);
 }
 
-// One warp per target leaf.  The target particles are taken 32 at a time; a chunk of m <= 16 (or <= 8)
-// targets is replicated over 2 (or 4) lane groups, each group walking every 2nd (4th) source record, and the
-// groups' sums are combined by shuffles at the end, so that small and ragged leaves keep the lanes busy.
+// One warp per work item.  A lane carries two targets, so that each record that it reads from shared memory serves
+// four pairs.  What bounds the kernel is the FP32 pipe (19 packed instructions per record and target, 1.96 Tpairs/s at
+// most) and the instructions around the pair loop: with one target per lane, stages of 32 records and a compensated
+// sum per stage, about half of the issued instructions were not the pairs'.  Two targets alone changed nothing; with
+// stages of 56 records (the three z-neighbours of a leaf of 30 are one stage), packed compensated sums of both targets
+// after every 24 records of a lane (chains no longer than before: the error is 0.9-1.0 of the earlier kernel's) and
+// 126 registers (4 CTAs per SM): 1M uniform 0.885 -> 0.82 ms, 2M on a surface 6.13 -> 5.5 ms, 200k in leaves of 49
+// 0.345 -> 0.28 ms.  Sums after every 16 records cost 4 % more, after every 64 give 2 % but a larger error.
+// The targets are taken 64, 32, 16 or 8 at a time (p2p_chunk); 32 (16, 8) targets occupy 16 (8, 4) lanes and are
+// replicated over 2 (4, 8) lane groups, each group walking every 2nd (4th, 8th) source record, and the groups' sums
+// are combined by shuffles at the end, so that small and ragged leaves keep the lanes busy.
 // The sources are walked as runs of contiguous records (one per neighbour column and z-adjacent group),
 // each split into stages of <= P2P32_STAGE records copied by one bulk copy into a ring of P2P32_NBUF buffers,
 // issued P2P32_NBUF - 1 stages ahead of the math.  Per stage the partial sums enter the target's (hi, lo)
@@ -366,7 +396,11 @@ __device__ __forceinline__ bool p2p_item(long long item, long long nleaves, cons
   return true;
 }
 
-__global__ void __launch_bounds__(P2P32_WARPS * 32, 7) p2p_fp32_kernel(
+// Targets of the next pass over the sources, of `left` that remain: a power of two with at least half of the 2 x 32
+// slots in use, and 33..48 as 32 and the rest.
+__device__ __forceinline__ int p2p_chunk(long long left) { return left > 48 ? 64 : left > 16 ? 32 : left > 8 ? 16 : 8; }
+
+__global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
     const long long *__restrict__ chunk_base, int whole, int isize, const long long *__restrict__ shard,
@@ -427,19 +461,27 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 7) p2p_fp32_kernel(
   for (int r = 0; r < R; ++r) {
     const float4 *pr = pq + (long long)r * N;
     const float4 *sr = src + (long long)r * P * 4;
-    for (long long tb = c0; tb < c1; tb += 32) {
-      const int m = (int)min(32LL, c1 - tb);
-      const int T = m <= 8 ? 8 : (m <= 16 ? 16 : 32);  // targets per lane group
-      const int G = 32 / T;                             // lane groups, each on every G-th record
+    for (long long tb = c0; tb < c1;) {
+      const int chunk = p2p_chunk(c1 - tb);
+      const int m = (int)min((long long)chunk, c1 - tb);
+      const int T = chunk / P2P32_TGT;  // lanes per group
+      const int G = 32 / T;             // lane groups, each on every G-th record
       const int tl = lane & (T - 1), g = lane / T;
-      const long long i = tb + tl;
-      const bool active = tl < m;
-      const float4 me = active ? pr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 mel = active ? plo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const long long self_slot = 2 * self_rec + (i - t0);  // the target's own slot in the record numbering
-      const float2 th_x = make_float2(me.x, me.x), th_y = make_float2(me.y, me.y), th_z = make_float2(me.z, me.z);
-      const float2 tl_x = make_float2(mel.x, mel.x), tl_y = make_float2(mel.y, mel.y), tl_z = make_float2(mel.z, mel.z);
-      float ph_hi = 0.f, ph_lo = 0.f, gx_hi = 0.f, gx_lo = 0.f, gy_hi = 0.f, gy_lo = 0.f, gz_hi = 0.f, gz_lo = 0.f;
+      Target32 tg[P2P32_TGT];
+      float tq[P2P32_TGT];
+      float2 hi[4], lo[4];  // compensated potential and force sums of both targets (.x, .y)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) hi[c] = lo[c] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < P2P32_TGT; ++u) {
+        const bool on = tl + u * T < m;
+        const float4 me = on ? pr[tb + tl + u * T] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 mel = on ? plo[tb + tl + u * T] : make_float4(0.f, 0.f, 0.f, 0.f);
+        tg[u] = {make_float2(me.x, me.x),   make_float2(me.y, me.y),   make_float2(me.z, me.z),
+                 make_float2(mel.x, mel.x), make_float2(mel.y, mel.y), make_float2(mel.z, mel.z)};
+        tq[u] = me.w;
+      }
+      const long long self_slot = 2 * self_rec + (tb + tl - t0);  // target 0's own slot in the record numbering
       // stage sequence: (run e, first record p, record count n); issue up to NBUF-1 stages ahead
       int ie = 0, ip = 0;  // next stage to issue
       int ce = 0, cp = 0;  // stage being computed
@@ -484,63 +526,59 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 7) p2p_fp32_kernel(
           return;
         }
         phase_bits ^= 1u << b;
-        float2 pv = make_float2(0.f, 0.f), ax = pv, ay = pv, az = pv;
         const float4 *s = buf[w][b];
-        if (rself[w][ce]) {
-          const int self_rel = (int)(self_slot - 2 * (rbase[w][ce] + cp));  // the target's slot in this stage
+        const bool own = rself[w][ce];
+        int self_rel[P2P32_TGT];
+#pragma unroll
+        for (int u = 0; u < P2P32_TGT; ++u)  // the target's slot in this stage
+          self_rel[u] = (int)(self_slot - 2 * (rbase[w][ce] + cp)) + u * T;
+        for (int k0 = g; k0 < cn; k0 += P2P32_FLUSH * G) {
+          const int k1 = min(cn, k0 + P2P32_FLUSH * G);
+          Sums32 acc[P2P32_TGT];
+#pragma unroll
+          for (int u = 0; u < P2P32_TGT; ++u) acc[u].pv = acc[u].ax = acc[u].ay = acc[u].az = make_float2(0.f, 0.f);
+          if (own) {
 #pragma unroll 2
-          for (int k = g; k < cn; k += G)
-            p2p_record<true>(s, k, self_rel, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv, ax, ay, az);
-        } else {
-          // two independent accumulator sets, so that consecutive records do not wait on each other's sums
-          float2 pv2 = make_float2(0.f, 0.f), ax2 = pv2, ay2 = pv2, az2 = pv2;
-          int k = g;
+            for (int k = k0; k < k1; k += G) p2p_record<true>(s, k, self_rel, tg, acc);
+          } else {
 #pragma unroll 2
-          for (; k + G < cn; k += 2 * G) {
-            p2p_record<false>(s, k, 0, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv, ax, ay, az);
-            p2p_record<false>(s, k + G, 0, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv2, ax2, ay2, az2);
+            for (int k = k0; k < k1; k += G) p2p_record<false>(s, k, self_rel, tg, acc);
           }
-          if (k < cn) p2p_record<false>(s, k, 0, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv, ax, ay, az);
-          pv = __fadd2_rn(pv, pv2);
-          ax = __fadd2_rn(ax, ax2);
-          ay = __fadd2_rn(ay, ay2);
-          az = __fadd2_rn(az, az2);
+          two_sum2(hi[0], lo[0], make_float2(acc[0].pv.x + acc[0].pv.y, acc[1].pv.x + acc[1].pv.y));
+          two_sum2(hi[1], lo[1], make_float2(acc[0].ax.x + acc[0].ax.y, acc[1].ax.x + acc[1].ax.y));
+          two_sum2(hi[2], lo[2], make_float2(acc[0].ay.x + acc[0].ay.y, acc[1].ay.x + acc[1].ay.y));
+          two_sum2(hi[3], lo[3], make_float2(acc[0].az.x + acc[0].az.y, acc[1].az.x + acc[1].az.y));
         }
-        two_sum(ph_hi, ph_lo, pv.x + pv.y);
-        two_sum(gx_hi, gx_lo, ax.x + ax.y);
-        two_sum(gy_hi, gy_lo, ay.x + ay.y);
-        two_sum(gz_hi, gz_lo, az.x + az.y);
         cp += cn;
         ++done;
         __syncwarp();  // every lane is done with buffer b before it is refilled
         issue();
       }
       // combine the lane groups that shared this chunk's targets
-      for (int off = T; off < 32; off <<= 1) {
-        float oh = __shfl_xor_sync(0xffffffffu, ph_hi, off), ol = __shfl_xor_sync(0xffffffffu, ph_lo, off);
-        two_sum(ph_hi, ph_lo, oh);
-        ph_lo += ol;
-        oh = __shfl_xor_sync(0xffffffffu, gx_hi, off);
-        ol = __shfl_xor_sync(0xffffffffu, gx_lo, off);
-        two_sum(gx_hi, gx_lo, oh);
-        gx_lo += ol;
-        oh = __shfl_xor_sync(0xffffffffu, gy_hi, off);
-        ol = __shfl_xor_sync(0xffffffffu, gy_lo, off);
-        two_sum(gy_hi, gy_lo, oh);
-        gy_lo += ol;
-        oh = __shfl_xor_sync(0xffffffffu, gz_hi, off);
-        ol = __shfl_xor_sync(0xffffffffu, gz_lo, off);
-        two_sum(gz_hi, gz_lo, oh);
-        gz_lo += ol;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        for (int off = T; off < 32; off <<= 1) {
+          const float2 oh = make_float2(__shfl_xor_sync(0xffffffffu, hi[c].x, off), __shfl_xor_sync(0xffffffffu, hi[c].y, off));
+          const float2 ol = make_float2(__shfl_xor_sync(0xffffffffu, lo[c].x, off), __shfl_xor_sync(0xffffffffu, lo[c].y, off));
+          two_sum2(hi[c], lo[c], oh);
+          lo[c] = __fadd2_rn(lo[c], ol);
+        }
+      if (g == 0) {
+#pragma unroll
+        for (int u = 0; u < P2P32_TGT; ++u) {
+          if (tl + u * T >= m) continue;
+          const long long j = (long long)r * N + tb + tl + u * T;
+          const double nq = -(double)tq[u];
+          double v[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = u == 0 ? (double)hi[c].x + (double)lo[c].x : (double)hi[c].y + (double)lo[c].y;
+          phi[j] += v[0];
+          fx[j] += nq * v[1];
+          fy[j] += nq * v[2];
+          fz[j] += nq * v[3];
+        }
       }
-      if (active && g == 0) {
-        const long long j = (long long)r * N + i;
-        const double tq = -(double)me.w;
-        phi[j] += (double)ph_hi + (double)ph_lo;
-        fx[j] += tq * ((double)gx_hi + (double)gx_lo);
-        fy[j] += tq * ((double)gy_hi + (double)gy_lo);
-        fz[j] += tq * ((double)gz_hi + (double)gz_lo);
-      }
+      tb += m;
     }
   }
 }
@@ -556,6 +594,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 7) p2p_fp32_kernel(
 //   charges of right-hand sides past R are zero.  Record order and runs are those of the single-RHS kernel.
 constexpr int MR_G = 4;
 constexpr int MR_REC = 5;  // float4 per record
+constexpr int MR_STAGE = 48;  // records per bulk-copy stage (32: 3.4 against 3.0 ms at 250k points x 16)
 
 __global__ void pack_records32_mrhs(long long N, int R, const long long *__restrict__ leaf_start,
                                     const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
@@ -640,8 +679,10 @@ __device__ __forceinline__ void p2p_record_mrhs(const float4 *__restrict__ s, in
   }
 }
 
-// The single-RHS kernel's walk (one warp per target leaf, runs of records in bulk-copy stages, lane groups for
-// small leaves, per-stage two-sums), with MR_G right-hand sides per pass over the sources.
+// One warp per work item and group of MR_G right-hand sides (grid.y): runs of records in bulk-copy stages, one target
+// per lane (two would need 64 accumulator registers more), lane groups for small leaves, per-stage two-sums.  With
+// the groups one after the other in a warp, 4,096 leaves of 61 gave 1.7 waves of long items: 3.7 -> 2.6 ms with the
+// groups on the grid, items of 32 targets and the longer stages (250k points x 16).
 __global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_mrhs_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
@@ -650,7 +691,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_mrhs_kernel(
     const float4 *__restrict__ src,
     double *__restrict__ phi, double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz,
     int *__restrict__ status) {
-  __shared__ __align__(128) float4 buf[P2P32_WARPS][P2P32_NBUF][MR_REC * P2P32_STAGE];
+  __shared__ __align__(128) float4 buf[P2P32_WARPS][P2P32_NBUF][MR_REC * MR_STAGE];
   __shared__ __align__(8) unsigned long long bar[P2P32_WARPS][P2P32_NBUF];
   __shared__ long long rbase[P2P32_WARPS][27];
   __shared__ int rcount[P2P32_WARPS][27];
@@ -701,7 +742,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_mrhs_kernel(
   }
   unsigned phase_bits = 0;
   const int G = (R + MR_G - 1) / MR_G;
-  for (int grp = 0; grp < G; ++grp) {
+  for (int grp = blockIdx.y; grp < G; grp += gridDim.y) {
     const float4 *sr = src + (long long)grp * P * MR_REC;
     for (long long tb = c0; tb < c1; tb += 32) {
       const int m = (int)min(32LL, c1 - tb);
@@ -726,7 +767,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_mrhs_kernel(
           p0 = 0;
         }
         if (e >= nr) return false;
-        n = min(P2P32_STAGE, rcount[w][e] - p0);
+        n = min(MR_STAGE, rcount[w][e] - p0);
         return true;
       };
       auto issue = [&]() {
@@ -844,7 +885,7 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     // work items (p2p_leaf_items per leaf): nleaves + N / item bounds their count
     const unsigned blocks = grid_for(L.n + c.N / c.p2p_item, P2P32_WARPS);
     B200_CUDA(record_event(c, 10));
-    p2p_fp32_mrhs_kernel<<<blocks, P2P32_WARPS * 32, 0, c.stream>>>(
+    p2p_fp32_mrhs_kernel<<<dim3(blocks, (c.R + MR_G - 1) / MR_G), P2P32_WARPS * 32, 0, c.stream>>>(
         c.R, c.N, L.n, c.d_leaf_start, c.d_leaf_nbr, variant, c.d_leaf_rank, c.d_rec_base, c.d_chunk_base, c.p2p_whole,
         c.p2p_item, shard, hi, lo, qt, src, c.d_phi, c.d_fx, c.d_fy, c.d_fz, c.d_status);
     B200_CUDA(record_event(c, 11));
