@@ -8,7 +8,7 @@
 // with x mapped to [-1,1] around the leaf centre (map_glob_loc, Src/Kernels/Interpolation/FInterpMapping.hpp:
 // 101-114; leaf centre FAbstractChebKernel.hpp:54-59).  Lagrange: FUnifInterpolator.hpp:340-549.
 // Every contraction is done one axis at a time (p^4 work per cell instead of p^6); leaves are handled one
-// warp each, parent cells one CTA each with one warp per child.
+// CTA (P2M) or warp (L2P) each, parent cells one CTA each with one warp per child.
 #include "common.cuh"
 
 namespace b200 {
@@ -16,11 +16,13 @@ namespace b200 {
 namespace {
 
 // Interpolation nodes of every built order (3..8) and basis (Chebyshev, Lagrange), and the Chebyshev values
-// T_o(node_j): read by P2M and L2P as constant-bank operands, so that the tables hold no registers.  Set per
-// device when a handle builds its tables (upload_basis_constants); every handle of an order and basis writes
-// the same values.
+// T_o(node_j): read by P2M and L2P as constant-bank operands, so that the tables hold no registers.  The same for
+// the child-to-parent interpolators of M2M and L2L, which are the same along every axis: one for the lower and one
+// for the upper child.  Set per device when a handle builds its tables (upload_basis_constants); every handle of an
+// order and basis writes the same values.
 __constant__ double c_roots[2][kMaxOrder - 2][kMaxOrder];      // [basis: 1 = Lagrange][p - 3][j]
 __constant__ double c_Tr[kMaxOrder - 2][kMaxOrder * kMaxOrder];  // [p - 3][o * p + j], Chebyshev
+__constant__ double c_S[2][kMaxOrder - 2][2][kMaxOrder * kMaxOrder];  // [basis][p - 3][child bit][n * p + m]
 
 // S_j(x) and dS_j/dx for j < p.  Chebyshev: 1/p + 2/p sum_o T_o(x) T_o(xbar_j), dT_o = o U_{o-1}.
 // Lagrange (equispaced nodes): prod_{m != j} (x - x_m) / (x_j - x_m) and its derivative.  Compile-time order
@@ -95,7 +97,10 @@ __device__ __forceinline__ void record_max(unsigned long long *slots, double mx)
 // M[nx,ny,nz] = sum_j q_j Sx_j[nx] Sy_j[ny] Sz_j[nz].  The threads first evaluate the 1-D weights of up to 64
 // particles (one each) into shared memory; then thread t < p^2 owns the node line (ny, nz) = (t % p, t / p)
 // and keeps its p sums over nx in registers: per particle one product q Sy Sz and p FMAs with the
-// broadcast Sx row, instead of three shared-memory reads per node and particle.
+// broadcast Sx row, instead of three shared-memory reads per node and particle.  Several right-hand sides share the
+// weights of a leaf of one chunk.  (Measured slower, 1M uniform, order 7, height 6: 128 threads, the weights along
+// rows of particles, two particles per load and two node lines per lane, 0.250 against 0.148 ms: 96 registers with
+// spills and three more barriers per leaf cost more than the halved shared-memory reads give.)
 constexpr int P2M_THREADS = 64;
 constexpr int L2P_WARPS = 2;  // L2P: leaves per CTA, one warp each (static shared memory <= 48 KB at order 8)
 
@@ -105,7 +110,7 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
     const long long *__restrict__ leaf_start, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, const double *__restrict__ q, double cx0, double cy0, double cz0, double leaf_w,
     double *__restrict__ M, unsigned long long *__restrict__ mmax) {
-  constexpr int p = P, nn = P * P * P, PX = (P + 1) & ~1;  // Sx rows padded to 16 bytes
+  constexpr int p = P, nn = P * P * P, PX = P <= 6 ? (P + 1) & ~1 : 10;  // Sx rows: 16-byte steps, spread over the banks
   __shared__ __align__(16) double Wx[P2M_THREADS][PX];
   __shared__ double Wy[P2M_THREADS][P], Wz[P2M_THREADS][P], Q[P2M_THREADS];
   const int t = threadIdx.x;
@@ -127,13 +132,15 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
         const long long i = b + t;
         const double pos[3] = {x[i], y[i], z[i]};
         double wv[P];
+        if (r == 0 || s1 - s0 > P2M_THREADS) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double a = ctr[d] - leaf_w / 2, bb = ctr[d] + leaf_w / 2;
-          basis_eval<P, LAGR>((2.0 * pos[d] - bb - a) / (bb - a), wv, nullptr);
-          double *dst = d == 0 ? Wx[t] : (d == 1 ? Wy[t] : Wz[t]);
+          for (int d = 0; d < 3; ++d) {
+            const double a = ctr[d] - leaf_w / 2, bb = ctr[d] + leaf_w / 2;
+            basis_eval<P, LAGR>((2.0 * pos[d] - bb - a) / (bb - a), wv, nullptr);
+            double *dst = d == 0 ? Wx[t] : (d == 1 ? Wy[t] : Wz[t]);
 #pragma unroll
-          for (int k = 0; k < p; ++k) dst[k] = wv[k];
+            for (int k = 0; k < p; ++k) dst[k] = wv[k];
+          }
         }
         Q[t] = q[(long long)r * N + i];
       }
@@ -160,86 +167,104 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
   }
 }
 
-// Copy NN doubles with T threads, all loads issued before the first store (one memory latency per copy
-// instead of one per element); ADD adds into dst instead of overwriting.
-template <int NN, int T, bool ADD = false>
-__device__ __forceinline__ void copy_block(double *dst, const double *__restrict__ src, int tid) {
-  constexpr int K = (NN + T - 1) / T;
-  double v[K], d[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int e = tid + k * T;
-    v[k] = e < NN ? src[e] : 0.0;
-    if (ADD) d[k] = e < NN ? dst[e] : 0.0;
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int e = tid + k * T;
-    if (e < NN) dst[e] = ADD ? d[k] + v[k] : v[k];
-  }
-}
-
 // ---- M2M / L2L: one warp per child ------------------------------------------------------------------
-// Each warp applies the child's three 1-D interpolators, one axis at a time, in its own shared-memory
-// buffers.  A lane owns whole lines along the axis: it loads the line's p values into registers and writes
-// the p results, with the p x p interpolator in registers.  M2M: the 8 children's contributions to the
-// parent are then added in child order (deterministic).
-template <int P, bool TRANSPOSE>
-__device__ __forceinline__ void warp_lines(const double *__restrict__ A, int d, const double *in, double *out,
-                                           int lane) {
-  constexpr int p = P, nl = P * P;
-  double a[P][P];
+// Each warp applies the child's three 1-D interpolators, one axis at a time, in place in its shared-memory block
+// (rows of p values padded to an odd length).  A lane owns whole lines along the axis: it loads the line's p values
+// into registers and writes the p results; the p x p interpolator is read as constant-bank operands, by a branch on
+// the child's bit of that axis.  (Loaded from global memory by every lane it cost 147 broadcast loads per child: the
+// load pipe was 75 % busy.)  M2M: the 8 children's contributions to the parent are then added in child order
+// (deterministic).  1M uniform, order 7, height 6, all levels: M2M 0.124 -> 0.087 ms, L2L 0.113 -> 0.072 ms.
+template <int P>
+struct Block {
+  static constexpr int PR = P | 1;             // row length
+  static constexpr int SIZE = P * P * PR;      // doubles
+  static __device__ __forceinline__ int at(int e) { return e / P * PR + e % P; }
+};
+
+template <int P, bool LAGR, bool TRANSPOSE, int D, int BIT>
+__device__ __forceinline__ void warp_lines_bit(const double *in, double *out, int lane) {
+  constexpr int p = P, nl = P * P, PR = Block<P>::PR;
+  constexpr int stride = D == 0 ? 1 : (D == 1 ? PR : PR * P);
+  constexpr int LN = (nl + 31) / 32;  // a lane's lines, together: each interpolator value is read once
+  const double *A = c_S[LAGR ? 1 : 0][P - 3][BIT];
+  int base[LN];
+  double v[LN][P];
 #pragma unroll
-  for (int i = 0; i < p; ++i)
-#pragma unroll
-    for (int m = 0; m < p; ++m) a[i][m] = TRANSPOSE ? A[m * p + i] : A[i * p + m];
-  const int stride = d == 0 ? 1 : (d == 1 ? p : p * p);
-  for (int l = lane; l < nl; l += 32) {
+  for (int u = 0; u < LN; ++u) {
+    const int l = lane + 32 * u;
     // first element of line l: the two other indices of the line, in increasing axis order
-    const int base = d == 0 ? l * p : (d == 1 ? (l % p) + (l / p) * p * p : l);
-    double v[P];
+    base[u] = D == 0 ? l * PR : (D == 1 ? (l % p) + (l / p) * PR * p : (l % p) + (l / p) * PR);
 #pragma unroll
-    for (int m = 0; m < p; ++m) v[m] = in[base + m * stride];
+    for (int m = 0; m < p; ++m) v[u][m] = l < nl ? in[base[u] + m * stride] : 0.0;
+  }
 #pragma unroll
-    for (int i = 0; i < p; ++i) {
-      double s = 0.0;
+  for (int i = 0; i < p; ++i) {
+    double s[LN];
 #pragma unroll
-      for (int m = 0; m < p; ++m) s += a[i][m] * v[m];
-      out[base + i * stride] = s;
-    }
+    for (int u = 0; u < LN; ++u) s[u] = 0.0;
+#pragma unroll
+    for (int m = 0; m < p; ++m)
+#pragma unroll
+      for (int u = 0; u < LN; ++u) s[u] += A[TRANSPOSE ? m * p + i : i * p + m] * v[u][m];
+#pragma unroll
+    for (int u = 0; u < LN; ++u)
+      if (lane + 32 * u < nl) out[base[u] + i * stride] = s[u];
   }
 }
+template <int P, bool LAGR, bool TRANSPOSE, int D>
+__device__ __forceinline__ void warp_lines(int child, const double *in, double *out, int lane) {
+  if ((child >> (2 - D)) & 1)
+    warp_lines_bit<P, LAGR, TRANSPOSE, D, 1>(in, out, lane);
+  else
+    warp_lines_bit<P, LAGR, TRANSPOSE, D, 0>(in, out, lane);
+}
 
-template <int P>
-__global__ void __launch_bounds__(256) m2m_kernel(int R, long long nparents, const int *__restrict__ child,
-                                                  const double *__restrict__ S, const double *__restrict__ Mc,
-                                                  double *__restrict__ Mp, unsigned long long *__restrict__ mmax) {
-  constexpr int p = P, nn = P * P * P;
+template <int P, bool LAGR>
+__global__ void __launch_bounds__(256, 2) m2m_kernel(int R, long long nparents, const int *__restrict__ child,
+                                                  const double *__restrict__ Mc, double *__restrict__ Mp,
+                                                  unsigned long long *__restrict__ mmax) {
+  constexpr int nn = P * P * P, K = (nn + 31) / 32, KP = (nn + 255) / 256;
+  using B = Block<P>;
   extern __shared__ double sh[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double *b0 = sh + (size_t)w * 2 * nn, *b1 = b0 + nn;  // per-warp buffers; b1 ends with the contribution
+  double *b = sh + (size_t)w * B::SIZE;  // the child's multipole, then its contribution
   const long long pc = blockIdx.x;
   const int ci = child[pc * 8 + w];
   for (int r = 0; r < R; ++r) {
+    double *out = Mp + (pc * R + r) * nn;
+    double old[KP];
     if (ci >= 0) {
-      copy_block<nn, 32>(b0, Mc + ((long long)ci * R + r) * nn, lane);
+      const double *src = Mc + ((long long)ci * R + r) * nn;
+      double v[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = lane + 32 * k < nn ? src[lane + 32 * k] : 0.0;
+#pragma unroll
+      for (int k = 0; k < KP; ++k) old[k] = threadIdx.x + 256 * k < nn ? out[threadIdx.x + 256 * k] : 0.0;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < nn) b[B::at(lane + 32 * k)] = v[k];
       __syncwarp();
-      warp_lines<P, false>(S + (w * 3 + 0) * p * p, 0, b0, b1, lane);
+      warp_lines<P, LAGR, false, 0>(w, b, b, lane);
       __syncwarp();
-      warp_lines<P, false>(S + (w * 3 + 1) * p * p, 1, b1, b0, lane);
+      warp_lines<P, LAGR, false, 1>(w, b, b, lane);
       __syncwarp();
-      warp_lines<P, false>(S + (w * 3 + 2) * p * p, 2, b0, b1, lane);
+      warp_lines<P, LAGR, false, 2>(w, b, b, lane);
     } else {
-      for (int e = lane; e < nn; e += 32) b1[e] = 0.0;
+#pragma unroll
+      for (int k = 0; k < KP; ++k) old[k] = threadIdx.x + 256 * k < nn ? out[threadIdx.x + 256 * k] : 0.0;
+      for (int e = lane; e < B::SIZE; e += 32) b[e] = 0.0;
     }
     __syncthreads();
     double mx = 0.0;
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int e = threadIdx.x + 256 * k;
+      if (e >= nn) continue;
       double s = 0.0;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) s += sh[(size_t)k * 2 * nn + nn + e];
-      const double v = Mp[(pc * R + r) * nn + e] + s;
-      Mp[(pc * R + r) * nn + e] = v;
+      for (int c = 0; c < 8; ++c) s += sh[(size_t)c * B::SIZE + B::at(e)];
+      const double v = old[k] + s;
+      out[e] = v;
       mx = fmax(mx, fabs(v));
     }
     if (mmax) record_max(mmax, mx);
@@ -247,30 +272,59 @@ __global__ void __launch_bounds__(256) m2m_kernel(int R, long long nparents, con
   }
 }
 
-template <int P>
-__global__ void __launch_bounds__(256) l2l_kernel(int R, long long nparents, const int *__restrict__ child,
-                                                  const double *__restrict__ S, const double *__restrict__ Lp,
-                                                  double *__restrict__ Lc) {
-  constexpr int p = P, nn = P * P * P;
+template <int P, bool LAGR>
+__global__ void __launch_bounds__(256, 2) l2l_kernel(int R, long long nparents, const int *__restrict__ child,
+                                                  const double *__restrict__ Lp, double *__restrict__ Lc) {
+  constexpr int nn = P * P * P, K = (nn + 31) / 32, KP = (nn + 255) / 256;
+  using B = Block<P>;
   extern __shared__ double sh[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double *par = sh;  // parent local
-  double *b0 = sh + nn + (size_t)w * 2 * nn, *b1 = b0 + nn;
+  double *b = sh + (size_t)(w + 1) * B::SIZE;
   const long long pc = blockIdx.x;
   const int ci = child[pc * 8 + w];
   for (int r = 0; r < R; ++r) {
+    const double *src = Lp + (pc * R + r) * nn;
+    double *out = Lc + ((long long)ci * R + r) * nn;
+    double v[KP], old[K];
+#pragma unroll
+    for (int k = 0; k < KP; ++k) v[k] = threadIdx.x + 256 * k < nn ? src[threadIdx.x + 256 * k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) old[k] = ci >= 0 && lane + 32 * k < nn ? out[lane + 32 * k] : 0.0;
     __syncthreads();
-    copy_block<nn, 256>(par, Lp + (pc * R + r) * nn, threadIdx.x);
+#pragma unroll
+    for (int k = 0; k < KP; ++k)
+      if (threadIdx.x + 256 * k < nn) par[B::at(threadIdx.x + 256 * k)] = v[k];
     __syncthreads();
     if (ci < 0) continue;
-    warp_lines<P, true>(S + (w * 3 + 0) * p * p, 0, par, b0, lane);
+    warp_lines<P, LAGR, true, 0>(w, par, b, lane);
     __syncwarp();
-    warp_lines<P, true>(S + (w * 3 + 1) * p * p, 1, b0, b1, lane);
+    warp_lines<P, LAGR, true, 1>(w, b, b, lane);
     __syncwarp();
-    warp_lines<P, true>(S + (w * 3 + 2) * p * p, 2, b1, b0, lane);
+    warp_lines<P, LAGR, true, 2>(w, b, b, lane);
     __syncwarp();
-    double *out = Lc + ((long long)ci * R + r) * nn;
-    copy_block<nn, 32, true>(out, b0, lane);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (lane + 32 * k < nn) out[lane + 32 * k] = old[k] + b[B::at(lane + 32 * k)];
+    __syncwarp();
+  }
+}
+
+// Copy NN doubles with T threads, all loads issued before the first store (one memory latency per copy
+// instead of one per element).
+template <int NN, int T>
+__device__ __forceinline__ void copy_block(double *dst, const double *__restrict__ src, int tid) {
+  constexpr int K = (NN + T - 1) / T;
+  double v[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int e = tid + k * T;
+    v[k] = e < NN ? src[e] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int e = tid + k * T;
+    if (e < NN) dst[e] = v[k];
   }
 }
 
@@ -359,12 +413,16 @@ __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
 
 }  // namespace
 
-b200fmm_status upload_basis_constants(const Context &c, const double *roots, const double *Tr) {
+b200fmm_status upload_basis_constants(const Context &c, const double *roots, const double *Tr, const double *S) {
   const int p = c.p;
   if (p < 3 || p > kMaxOrder) return B200FMM_OK;  // no P2M / L2P kernel is built for this order
   const int lag = c.cfg.kernel == B200FMM_LAGRANGE ? 1 : 0;
   B200_CUDA(cudaMemcpyToSymbol(c_roots, roots, sizeof(double) * p,
                                sizeof(double) * ((size_t)(lag * (kMaxOrder - 2) + p - 3) * kMaxOrder)));
+  // S [8 children][3 axes][p][p]: children 0 and 4 differ in the bit of axis 0
+  for (int bit = 0; bit < 2; ++bit)
+    B200_CUDA(cudaMemcpyToSymbol(c_S, S + (size_t)bit * 4 * 3 * p * p, sizeof(double) * p * p,
+                                 sizeof(double) * ((size_t)((lag * (kMaxOrder - 2) + p - 3) * 2 + bit) * kMaxOrder * kMaxOrder)));
   if (!lag)
     B200_CUDA(cudaMemcpyToSymbol(c_Tr, Tr, sizeof(double) * p * p, sizeof(double) * (size_t)(p - 3) * kMaxOrder * kMaxOrder));
   return B200FMM_OK;
@@ -402,13 +460,15 @@ b200fmm_status run_m2m(Context &c, int level) {
   if (level < 2 || level >= c.H - 1) return fail(B200FMM_ERR_INVALID, "m2m: parent level must be in [2, height-2]");
   const Level &P = c.lv[level], &C = c.lv[level + 1];
   if (P.n == 0) return B200FMM_OK;
-  const size_t sh = sizeof(double) * 16 * c.nn;
+  const bool lagr = c.cfg.kernel == B200FMM_LAGRANGE;
   unsigned long long *mmax = c.mmax_out ? c.mmax_out + (size_t)level * kMmaxSlots : nullptr;
 #define B200_M2M(PV)                                                                                        \
-  case PV:                                                                                                  \
-    B200_CUDA(cudaFuncSetAttribute(m2m_kernel<PV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));   \
-    m2m_kernel<PV><<<(unsigned)P.n, 256, sh, c.stream>>>(c.R, P.n, P.child, c.d_S, C.M, P.M, mmax);         \
-    break;
+  case PV: {                                                                                                \
+    constexpr int sh = (int)sizeof(double) * 8 * Block<PV>::SIZE;                                           \
+    auto kernel = lagr ? m2m_kernel<PV, true> : m2m_kernel<PV, false>;                                      \
+    kernel<<<(unsigned)P.n, 256, sh, c.stream>>>(c.R, P.n, P.child, C.M, P.M, mmax);                        \
+    break;                                                                                                  \
+  }
   switch (c.p) {
     B200_M2M(3) B200_M2M(4) B200_M2M(5) B200_M2M(6) B200_M2M(7) B200_M2M(8)
     default: return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
@@ -423,12 +483,14 @@ b200fmm_status run_l2l(Context &c, int level) {
   if (level < 2 || level >= c.H - 1) return fail(B200FMM_ERR_INVALID, "l2l: parent level must be in [2, height-2]");
   const Level &P = c.lv[level], &C = c.lv[level + 1];
   if (P.n == 0) return B200FMM_OK;
-  const size_t sh = sizeof(double) * 17 * c.nn;
+  const bool lagr = c.cfg.kernel == B200FMM_LAGRANGE;
 #define B200_L2L(PV)                                                                                        \
-  case PV:                                                                                                  \
-    B200_CUDA(cudaFuncSetAttribute(l2l_kernel<PV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));   \
-    l2l_kernel<PV><<<(unsigned)P.n, 256, sh, c.stream>>>(c.R, P.n, P.child, c.d_S, P.L, C.L);               \
-    break;
+  case PV: {                                                                                                \
+    constexpr int sh = (int)sizeof(double) * 9 * Block<PV>::SIZE;                                           \
+    auto kernel = lagr ? l2l_kernel<PV, true> : l2l_kernel<PV, false>;                                      \
+    kernel<<<(unsigned)P.n, 256, sh, c.stream>>>(c.R, P.n, P.child, P.L, C.L);                              \
+    break;                                                                                                  \
+  }
   switch (c.p) {
     B200_L2L(3) B200_L2L(4) B200_L2L(5) B200_L2L(6) B200_L2L(7) B200_L2L(8)
     default: return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
