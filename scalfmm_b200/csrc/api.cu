@@ -113,19 +113,6 @@ b200fmm_status need_particles(Context &c) {
   return B200FMM_OK;
 }
 
-b200fmm_status zero_state(Context &c) {
-  for (int l = 2; l < c.H; ++l) {
-    const size_t bytes = sizeof(double) * (size_t)c.lv[l].n * c.R * c.nn;
-    if (bytes) {
-      B200_CUDA(cudaMemsetAsync(c.lv[l].M, 0, bytes, c.stream));
-      B200_CUDA(cudaMemsetAsync(c.lv[l].L, 0, bytes, c.stream));
-    }
-  }
-  const size_t pb = sizeof(double) * (size_t)c.N * c.R;
-  for (double *p : {c.d_phi, c.d_fx, c.d_fy, c.d_fz}) B200_CUDA(cudaMemsetAsync(p, 0, pb, c.stream));
-  return B200FMM_OK;
-}
-
 b200fmm_status record(Context &c, int k) {
   B200_CUDA(record_event(c, k));
   return B200FMM_OK;
@@ -324,8 +311,7 @@ b200fmm_status b200fmm_set_particles(b200fmm_handle h, long long n, const double
   B200_CUDA(cudaEventRecord(c.ev[14], c.stream));
   b200fmm_status st = build_tree(c, x, y, z, q, on_device != 0);
   if (st != B200FMM_OK) return st;
-  B200_CHECK(zero_state(c));  // a new tree starts from zero expansions and results
-  c.state_zero = true;
+  c.state_zero = true;  // a new tree starts from zero expansions and results
   // the FP64 M2L's per-tree tables for dense operators need a count from the device: it travels under the wait below
   const bool dense64 = c.cfg.precision == B200FMM_FP64 && c.cfg.kernel != B200FMM_CHEB_SYM;
   int *dense_first = (int *)(c.h_pinned + 64);
@@ -354,7 +340,7 @@ b200fmm_status b200fmm_reset_expansions(b200fmm_handle h) {
   Context &c = *h;
   B200_CHECK(need_particles(c));
   B200_CHECK(set_device(c));
-  B200_CHECK(zero_state(c));
+  B200_CHECK(clear_state(c));
   c.state_zero = true;
   return B200FMM_OK;
 }
@@ -381,7 +367,7 @@ static b200fmm_status execute_body(Context &c, unsigned ops) {
   const int LL = c.H - 1;
   B200_CHECK(record(c, 0));
   // skipped right after set_particles, which zeroed them; always part of a captured graph
-  if (!c.state_zero || c.capturing) B200_CHECK(zero_state(c));
+  if (!c.state_zero || c.capturing) B200_CHECK(clear_state(c));
   c.state_zero = false;
   // MIXED records the multipole maxima during a full upward pass for the tensor-core M2L
   c.mmax_out = nullptr;

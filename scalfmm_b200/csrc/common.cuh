@@ -156,13 +156,12 @@ struct Context {
   bool last_was_graph = false;            // the last execute() replayed the graph (only its total is timed)
 
   // grow-only buffers of the tree build (capacities in elements)
-  size_t cap_N = 0, cap_leaf = 0, cap_sort = 0, cap_cnt = 0, cap_stage = 0, cap_scan = 0;
+  size_t cap_N = 0, cap_leaf = 0, cap_sort = 0, cap_cnt = 0, cap_stage = 0, cap_flags = 0;
   unsigned long long *d_sortk = nullptr;  // [2N] radix-sort keys (ping-pong)
   int *d_sortv = nullptr;                 // [2N] radix-sort values
-  long long *d_flags = nullptr;           // [2(N+1)] head flags and their scan
-  unsigned *d_cnt = nullptr;              // radix histograms and offsets
+  long long *d_flags = nullptr;           // block counts of the compactions
+  unsigned *d_cnt = nullptr;              // radix histograms
   double *d_stage = nullptr;              // host input staged on the device
-  long long *d_scan = nullptr;            // scan block sums
   int *d_err = nullptr;                   // domain error flag; from byte 16 the cell count of each level
   long long *h_pinned = nullptr;          // small pinned host buffer for counts
   int tree_gen = 0;                       // bumped whenever a tree buffer moves
@@ -216,6 +215,21 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
                           bool on_device);
 b200fmm_status upload_charges(Context &c, const double *q, bool on_device);
 void free_tree(Context &c);
+b200fmm_status clear_state(Context &c);  // zero expansions and results
+// Clears of many buffers (16-byte aligned, whole 8-byte words) to zeros or ones in one launch.
+constexpr int kClearMax = 4 * kMaxHeight + 4;
+struct ClearArgs {
+  unsigned long long *p[kClearMax];
+  long long n[kClearMax];
+  unsigned first[kClearMax + 1];
+  unsigned char ones[kClearMax];
+  int count;
+};
+struct ClearList {
+  ClearArgs a{};
+  void add(void *p, size_t bytes, bool ones);
+  b200fmm_status launch(cudaStream_t s);
+};
 // interp.cu
 // the interpolation nodes, Chebyshev values and child-to-parent interpolators of the handle's order into the
 // device's constant tables
