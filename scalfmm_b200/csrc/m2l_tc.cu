@@ -1726,6 +1726,7 @@ struct PackLevels {
   long long pos0[kMaxHeight + 1];       // first grid position of each level (rhs, parity, z, y, x)
   int HX[kMaxHeight], HY[kMaxHeight], HZ[kMaxHeight], side[kMaxHeight];
   const int *grid[kMaxHeight];          // dense cell grid of the level: cell index or -1
+  const int *ccell[kMaxHeight];         // a compacted level: the cell of each row (-1: none) instead of the grid
   __half *hi[kMaxHeight], *lo[kMaxHeight];
   double scale_l[kMaxHeight];           // 2 / cell width
 };
@@ -1742,33 +1743,54 @@ __global__ void absmax_levels_kernel(const __grid_constant__ PackLevels L, unsig
   if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(amax + l, (unsigned long long)__double_as_longlong(m));
 }
 
-// every grid position of levels [l0, l1]: the scaled multipole of its cell, split into FP16 hi + lo, or
-// zeros where there is no cell (and in the K padding), so that the buffers need no clearing
-__global__ void pack_levels_kernel(const __grid_constant__ PackLevels L, int R, int nn, int KP,
-                                   const double *__restrict__ scal) {
-  const long long p = blockIdx.x + L.pos0[L.l0];
+// every grid position (compacted levels: row) of levels [l0, l1]: the scaled multipole of its cell, split into FP16
+// hi + lo, or zeros where there is no cell (and in the K padding), so that the buffers need no clearing.  A warp per
+// position, 16-byte stores of zeros, two values per lane otherwise: bound by the bytes written.  With a block of 128
+// threads per position and two-byte stores, the 300,000 mostly empty positions of a 2M-point surface at height 7
+// (order 6, 268 MB) took 0.31 ms, now 0.08.
+constexpr int PACK_WARPS = 4;
+__global__ void __launch_bounds__(32 * PACK_WARPS) pack_levels_kernel(const __grid_constant__ PackLevels L, int R,
+                                                                      int nn, int KP, const double *__restrict__ scal) {
+  const int lane = threadIdx.x & 31;
+  const long long p = (long long)blockIdx.x * PACK_WARPS + (threadIdx.x >> 5) + L.pos0[L.l0];
+  if (p >= L.pos0[L.l1 + 1]) return;
   int l = L.l0;
   while (l < L.l1 && p >= L.pos0[l + 1]) ++l;
-  long long r = p - L.pos0[l];
-  const long long base = r * KP;
-  const int hx = (int)(r % L.HX[l]);
-  r /= L.HX[l];
-  const int hy = (int)(r % L.HY[l]);
-  r /= L.HY[l];
-  const int hz = (int)(r % L.HZ[l]);
-  const int r8 = (int)(r / L.HZ[l]);
-  const int par = r8 & 7, rhs = r8 >> 3;
-  const int gx = 2 * hx + ((par >> 2) & 1), gy = 2 * hy + ((par >> 1) & 1), gz = 2 * hz + (par & 1);
-  const int side = L.side[l];
-  int cell = -1;
-  if (gx < side && gy < side && gz < side) cell = L.grid[l][((long long)gz * side + gy) * side + gx];
+  const long long row = p - L.pos0[l];
+  int cell = -1, rhs = 0;
+  if (L.ccell[l]) {
+    cell = L.ccell[l][row];
+  } else {
+    long long r = row;
+    const int hx = (int)(r % L.HX[l]);
+    r /= L.HX[l];
+    const int hy = (int)(r % L.HY[l]);
+    r /= L.HY[l];
+    const int hz = (int)(r % L.HZ[l]);
+    const int r8 = (int)(r / L.HZ[l]);
+    const int par = r8 & 7;
+    rhs = r8 >> 3;
+    const int gx = 2 * hx + ((par >> 2) & 1), gy = 2 * hy + ((par >> 1) & 1), gz = 2 * hz + (par & 1);
+    const int side = L.side[l];
+    if (gx < side && gy < side && gz < side) cell = L.grid[l][((long long)gz * side + gy) * side + gx];
+  }
+  __half *hi = L.hi[l] + row * KP, *lo = L.lo[l] + row * KP;
+  if (cell < 0) {
+    for (int n = 8 * lane; n < KP; n += 256) {
+      *reinterpret_cast<uint4 *>(hi + n) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4 *>(lo + n) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    return;
+  }
   const double s = scal[2 * l];
-  const double *m = cell >= 0 ? L.M[l] + ((long long)cell * R + rhs) * nn : nullptr;
-  for (int n = threadIdx.x; n < KP; n += blockDim.x) {
-    const double a = (m && n < nn) ? m[n] * s : 0.0;
-    const __half h = __double2half(a);
-    L.hi[l][base + n] = h;
-    L.lo[l][base + n] = __double2half(a - (double)__half2float(h));
+  const double *m = L.M[l] + ((long long)cell * R + rhs) * nn;
+#pragma unroll 2
+  for (int n = 2 * lane; n < KP; n += 64) {
+    const double a = n < nn ? m[n] * s : 0.0, b = n + 1 < nn ? m[n + 1] * s : 0.0;
+    const __half ha = __double2half(a), hb = __double2half(b);
+    *reinterpret_cast<__half2 *>(hi + n) = __halves2half2(ha, hb);
+    *reinterpret_cast<__half2 *>(lo + n) = __halves2half2(__double2half(a - (double)__half2float(ha)),
+                                                          __double2half(b - (double)__half2float(hb)));
   }
 }
 
@@ -1781,51 +1803,70 @@ __device__ __forceinline__ int key_parity(long long key, int &ix, int &iy, int &
   morton_decode3(key, ix, iy, iz);
   return ((ix & 1) << 2) | ((iy & 1) << 1) | (iz & 1);
 }
-__global__ void __launch_bounds__(1024) cgroup_count_kernel(const long long *__restrict__ keys, long long n,
-                                                            int *__restrict__ gcnt) {
+// The groups of the placed levels, one after the other: every kernel serves all levels in one launch.
+struct CGroups {
+  const long long *keys[kMaxHeight];
+  long long n[kMaxHeight];
+  int g0[kMaxHeight + 1];  // first group of each level (levels that are not placed have none)
+  int l0, l1;
+};
+__device__ __forceinline__ int cgroup_level(const CGroups &G, int g) {
+  int l = G.l0;
+  while (l < G.l1 && g >= G.g0[l + 1]) ++l;
+  return l;
+}
+__global__ void __launch_bounds__(1024) cgroup_count_kernel(const __grid_constant__ CGroups G, int *__restrict__ gcnt) {
   __shared__ int cnt[8];
   if (threadIdx.x < 8) cnt[threadIdx.x] = 0;
   __syncthreads();
-  const long long i = blockIdx.x * 1024LL + threadIdx.x;
-  if (i < n) {
+  const int l = cgroup_level(G, blockIdx.x);
+  const long long i = (blockIdx.x - G.g0[l]) * 1024LL + threadIdx.x;
+  if (i < G.n[l]) {
     int ix, iy, iz;
-    atomicAdd(&cnt[key_parity(keys[i], ix, iy, iz)], 1);
+    atomicAdd(&cnt[key_parity(G.keys[l][i], ix, iy, iz)], 1);
   }
   __syncthreads();
   if (threadIdx.x < 8) gcnt[blockIdx.x * 8 + threadIdx.x] = cnt[threadIdx.x];
 }
-// one warp per parity: the group counts become exclusive offsets in place, the total goes to tot[p]
-__global__ void __launch_bounds__(256) cgroup_scan_kernel(int ngroups, int *__restrict__ gcnt, int *__restrict__ tot) {
-  const int p = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// a CTA per level, one warp per parity: the group counts become exclusive offsets in place, the total goes to
+// tot[level][p]
+__global__ void __launch_bounds__(256) cgroup_scan_kernel(const __grid_constant__ CGroups G, int *__restrict__ gcnt,
+                                                          int *__restrict__ tot) {
+  const int l = blockIdx.x, p = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int run = 0;
-  for (int g0 = 0; g0 < ngroups; g0 += 32) {
-    const int g = g0 + lane;
-    const int v = g < ngroups ? gcnt[g * 8 + p] : 0;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+  if (l >= G.l0 && l <= G.l1)
+    for (int g0 = G.g0[l]; g0 < G.g0[l + 1]; g0 += 32) {
+      const int g = g0 + lane;
+      const int v = g < G.g0[l + 1] ? gcnt[g * 8 + p] : 0;
+      int x = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (g < G.g0[l + 1]) gcnt[g * 8 + p] = run + x - v;
+      run += __shfl_sync(0xffffffffu, x, 31);
     }
-    if (g < ngroups) gcnt[g * 8 + p] = run + x - v;
-    run += __shfl_sync(0xffffffffu, x, 31);
-  }
-  if (lane == 0) tot[p] = run;
+  if (lane == 0) tot[l * 8 + p] = run;
 }
 struct CPlace {
   int blk0[9];  // first 128-row block of each parity (placement), or first Y chunk of each parity (cclear)
   int HX, HY;
 };
 // rowmap (optional): [parity][position] -> the cell's row counted from its parity's first block
-__global__ void __launch_bounds__(1024) cgroup_place_kernel(const long long *__restrict__ keys, long long n,
-                                                            const __grid_constant__ CPlace C,
-                                                            const int *__restrict__ goff, int *__restrict__ crow,
-                                                            int *__restrict__ ccell, int *__restrict__ rowmap,
-                                                            long long plane) {
+struct CPlaceLevels {
+  CPlace C[kMaxHeight];
+  long long plane[kMaxHeight];
+  int *crow[kMaxHeight], *ccell[kMaxHeight], *rowmap[kMaxHeight];
+};
+__global__ void __launch_bounds__(1024) cgroup_place_kernel(const __grid_constant__ CGroups G,
+                                                            const __grid_constant__ CPlaceLevels L,
+                                                            const int *__restrict__ goff) {
   __shared__ int wcnt[32][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long i = blockIdx.x * 1024LL + threadIdx.x;
+  const int l = cgroup_level(G, blockIdx.x);
+  const long long i = (blockIdx.x - G.g0[l]) * 1024LL + threadIdx.x;
   int ix = 0, iy = 0, iz = 0, par = -1;
-  if (i < n) par = key_parity(keys[i], ix, iy, iz);
+  if (i < G.n[l]) par = key_parity(G.keys[l][i], ix, iy, iz);
   const unsigned same = __match_any_sync(0xffffffffu, par);
   const int rk = __popc(same & ((1u << lane) - 1u));  // earlier lanes of this warp with the same parity
   (&wcnt[0][0])[threadIdx.x & 255] = 0;
@@ -1836,11 +1877,12 @@ __global__ void __launch_bounds__(1024) cgroup_place_kernel(const long long *__r
   int before = 0;
   for (int w = 0; w < warp; ++w) before += wcnt[w][par];
   const int prow = goff[blockIdx.x * 8 + par] + before + rk;
+  const CPlace &C = L.C[l];
   const int row = C.blk0[par] * 128 + prow;
   const int pos = ((iz >> 1) * C.HY + (iy >> 1)) * C.HX + (ix >> 1);
-  crow[row] = (par << 28) | pos;
-  ccell[row] = (int)i;
-  if (rowmap) rowmap[par * plane + pos] = prow;
+  L.crow[l][row] = (par << 28) | pos;
+  L.ccell[l][row] = (int)i;
+  if (L.rowmap[l]) L.rowmap[l][par * L.plane[l] + pos] = prow;
 }
 // Busy masks of the compacted blocks of every compacted level (one CTA of 128 threads per block, blocks
 // numbered across levels from b0): bit e set when the source of some row under transfer vector e is a cell,
@@ -1898,22 +1940,6 @@ __global__ void cclear_kernel(const int *__restrict__ crow, long long plane, con
     dh[0] = dh[1] = dl[0] = dl[1] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
-// the compacted multipoles of one evaluation: row -> its cell's multipole scaled and split as pack_levels does
-__global__ void pack_compact_kernel(const int *__restrict__ ccell, const double *__restrict__ M, int nn, int KP,
-                                    const double *__restrict__ scal_l, __half *__restrict__ hi,
-                                    __half *__restrict__ lo) {
-  const long long row = blockIdx.x;
-  const int cell = ccell[row];
-  const double s = *scal_l;
-  const double *m = cell >= 0 ? M + (long long)cell * nn : nullptr;
-  for (int n = threadIdx.x; n < KP; n += blockDim.x) {
-    const double a = (m && n < nn) ? m[n] * s : 0.0;
-    const __half h = __double2half(a);
-    hi[row * KP + n] = h;
-    lo[row * KP + n] = __double2half(a - (double)__half2float(h));
-  }
-}
-
 // 2^sA with sA chosen so that max|M| * 2^sA ~ 2^14, and the epilogue factor scale_l * 2^-(sA + shift)
 // with shift the operators' own pre-scale exponent (SB for the dense K, sV + sU - sY for the low-rank
 // factors).  One thread per level of [l0, l1]; max|M| of level l is the largest of amax[l * nslots + s].
@@ -2630,10 +2656,18 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
   const unsigned mask = ymask | tmask;
   // per-parity counts of every placed level, in groups of 1024 cells
   int cnt[kMaxHeight][8] = {};
-  long long g0[kMaxHeight + 1] = {};
+  CGroups G{};
+  G.l0 = 2;
+  G.l1 = LL;
+  long long ng = 0;
   if (mask) {
-    for (int l = 2; l <= LL; ++l) g0[l + 1] = g0[l] + (((mask >> l) & 1u) ? (c.lv[l].n + 1023) / 1024 : 0);
-    const long long ng = g0[LL + 1];
+    for (int l = 2; l <= LL; ++l) {
+      G.keys[l] = c.lv[l].keys;
+      G.n[l] = c.lv[l].n;
+      G.g0[l] = (int)ng;
+      ng += ((mask >> l) & 1u) ? (c.lv[l].n + 1023) / 1024 : 0;
+      G.g0[l + 1] = (int)ng;
+    }
     if (t.cgrp_cap < 8 * ng) {
       if (t.cgrp) cudaFree(t.cgrp);
       t.cgrp = nullptr;
@@ -2642,20 +2676,18 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
       t.cgrp_cap = 8 * ng;
     }
     if (!t.ccnt) B200_CUDA(cudaMalloc(&t.ccnt, sizeof(int) * kMaxHeight * 8));
-    B200_CUDA(cudaMemsetAsync(t.ccnt, 0, sizeof(int) * kMaxHeight * 8, c.stream));
-    for (int l = 2; l <= LL; ++l)
-      if ((mask >> l) & 1u) {
-        const int ngl = (int)(g0[l + 1] - g0[l]);
-        cgroup_count_kernel<<<ngl, 1024, 0, c.stream>>>(c.lv[l].keys, c.lv[l].n, t.cgrp + 8 * g0[l]);
-        cgroup_scan_kernel<<<1, 256, 0, c.stream>>>(ngl, t.cgrp + 8 * g0[l], t.ccnt + 8 * l);
-        c.launches += 2;
-      }
+    cgroup_count_kernel<<<(unsigned)ng, 1024, 0, c.stream>>>(G, t.cgrp);
+    cgroup_scan_kernel<<<kMaxHeight, 256, 0, c.stream>>>(G, t.cgrp, t.ccnt);
+    c.launches += 2;
+    B200_CUDA(cudaGetLastError());
     B200_CUDA(cudaMemcpyAsync(cnt, t.ccnt, sizeof(cnt), cudaMemcpyDeviceToHost, c.stream));
     B200_CUDA(cudaStreamSynchronize(c.stream));
   }
   // blocks of every placed level (an even count per parity for CTA pairs).  A level compacted in both products
   // (low rank) stores its Y by compacted row when the largest parity's rows fit the grid layout's rows.
-  CPlace Cl[kMaxHeight] = {};
+  CPlaceLevels pl{};
+  CPlace(&Cl)[kMaxHeight] = pl.C;
+  ClearList clear;
   int ypr[kMaxHeight] = {};
   for (int l = 2; l <= LL; ++l) {
     if (!((mask >> l) & 1u)) continue;
@@ -2723,18 +2755,18 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
       B200_CUDA(cudaMalloc(&t.ccell[l], sizeof(int) * rows));
       t.ccap[l] = rows;
     }
-    B200_CUDA(cudaMemsetAsync(t.crow[l], 0xFF, sizeof(int) * rows, c.stream));
-    B200_CUDA(cudaMemsetAsync(t.ccell[l], 0xFF, sizeof(int) * rows, c.stream));
+    clear.add(t.crow[l], sizeof(int) * rows, true);
+    clear.add(t.ccell[l], sizeof(int) * rows, true);
     int *rmap = nullptr;
     if (ypr[l] > 0) {
       if (!t.rowmap[l]) B200_CUDA(cudaMalloc(&t.rowmap[l], sizeof(int) * 8 * plane));
       rmap = t.rowmap[l];
-      B200_CUDA(cudaMemsetAsync(rmap, 0xFF, sizeof(int) * 8 * plane, c.stream));
+      clear.add(rmap, sizeof(int) * 8 * plane, true);
     }
-    const int ngl = (int)(g0[l + 1] - g0[l]);
-    cgroup_place_kernel<<<ngl, 1024, 0, c.stream>>>(c.lv[l].keys, c.lv[l].n, C, t.cgrp + 8 * g0[l], t.crow[l],
-                                                    t.ccell[l], rmap, plane);
-    ++c.launches;
+    pl.plane[l] = plane;
+    pl.crow[l] = t.crow[l];
+    pl.ccell[l] = t.ccell[l];
+    pl.rowmap[l] = rmap;
     t.crows[l] = (int)rows;
     P.lv[l].crow = t.crow[l];
     P.lv[l].ccell = t.ccell[l];
@@ -2766,6 +2798,12 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
       for (int p = 0; p <= 8; ++p) Y.cblk0[l][p] = C.blk0[p];
       Y.ypr[l] = ypr[l];
     }
+  }
+  if (ng > 0) {
+    B200_CHECK(clear.launch(c.stream));
+    cgroup_place_kernel<<<(unsigned)ng, 1024, 0, c.stream>>>(G, pl, t.cgrp);
+    c.launches += 2;
+    B200_CUDA(cudaGetLastError());
   }
   // first-product items (low rank), finest level first
   if (t.lr) {
@@ -2902,11 +2940,12 @@ b200fmm_status run_m2l_tc(Context &c, int level) {
       L.HZ[l] = t->HZ[l];
       L.side[l] = 1 << l;
       L.grid[l] = c.lv[l].grid;
-      L.hi[l] = t->Ahi[l];
-      L.lo[l] = t->Alo[l];
-      L.scale_l[l] = 2.0 / (c.cfg.box_width / (double)(1LL << l));
       const bool compact = t->lr && ((t->yparams->compact_levels >> l) & 1u);
-      L.pos0[l + 1] = L.pos0[l] + (compact ? 0LL : 8LL * c.R * t->HZ[l] * t->HY[l] * t->HX[l]);
+      L.ccell[l] = compact ? t->ccell[l] : nullptr;
+      L.hi[l] = compact ? t->Chi[l] : t->Ahi[l];
+      L.lo[l] = compact ? t->Clo[l] : t->Alo[l];
+      L.scale_l[l] = 2.0 / (c.cfg.box_width / (double)(1LL << l));
+      L.pos0[l + 1] = L.pos0[l] + (compact ? t->crows[l] : 8LL * c.R * t->HZ[l] * t->HY[l] * t->HX[l]);
     }
     const int shift = t->lr ? t->lr_shift : SB;
     if (c.mmax_ready) {
@@ -2920,17 +2959,11 @@ b200fmm_status run_m2l_tc(Context &c, int level) {
       ++c.launches;
     }
     if (L.pos0[l1 + 1] > 0) {
-      pack_levels_kernel<<<(unsigned)L.pos0[l1 + 1], 128, 0, c.stream>>>(L, c.R, c.nn, t->KP, t->scal);
+      pack_levels_kernel<<<grid_for(L.pos0[l1 + 1], PACK_WARPS), 32 * PACK_WARPS, 0, c.stream>>>(L, c.R, c.nn, t->KP,
+                                                                                                t->scal);
       ++c.launches;
     }
     ++c.launches;
-    if (t->lr)
-      for (int l = l0; l <= l1; ++l)
-        if (((t->yparams->compact_levels >> l) & 1u) && t->crows[l] > 0) {
-          pack_compact_kernel<<<(unsigned)t->crows[l], 128, 0, c.stream>>>(t->ccell[l], c.lv[l].M, c.nn, t->KP,
-                                                                           t->scal + 2 * l, t->Chi[l], t->Clo[l]);
-          ++c.launches;
-        }
   }
   // units are ordered by level, finest first: levels [l0, l1] are one contiguous range
   TcParams &P = *t->params;
