@@ -122,7 +122,6 @@ struct __align__(64) TcParams {
   int nbuf;  // TMEM accumulators: 2 (alternating per segment) when 2 * NP columns fit, else 1
   int stage_bytes;
   signed char off[8][189][3];
-  short slot[8][189];
   int *status;
   // per tile (level, parity, bz, by, bx): 6 words, bit e set when transfer vector e has an occupied source
   // box; bit 31 of word 5 set when the tile has an occupied target cell
@@ -140,6 +139,16 @@ struct __align__(64) TcParams {
   // target shard (or null): [2 + 2 l, 3 + 2 l] hold level l's owned cells [a, b); units without one do no work
   const long long *shard;
 };
+// What the kernels that build a tree's tables need of TcParams: passing all of it (13 KB of kernel parameters) cost
+// the host about 5 us per launch.
+struct TcTree {
+  TcLevel lv[kMaxHeight];
+  const IListTable *itab;
+  const unsigned *busy, *cbusy;
+  int l0, l1, pair;
+  const long long *shard;
+};
+
 // What the producer and the MMA issuers need of transfer vector e of target parity c: the A box's
 // coordinates (offset of the source tile in half-grid cells; outer coordinate ya + rhs * (ycht or 8)), the B
 // box's outer coordinate ub, and in the low-rank form the slot's 16-wide rank chunks nk.  Dense: ya = source
@@ -393,27 +402,10 @@ __device__ __forceinline__ void take_registers() {
   if constexpr (SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_HIGH));
 }
 
-// The source box of transfer vector e for an item: parity grid sp, half-grid origin (ox, oy, oz), operator
-// slot.  Every warp role derives the same box, and skips the transfer vectors whose source box is empty
-// (those A tiles are all zero) and the items whose target tile is empty, so that sparse trees (surface or
-// clustered distributions) cost only their occupied tiles.
-struct SrcBox {
-  int sp, ox, oy, oz, slot;
-};
-// bz: the target tile's z index (an item's tile, or in CTA pairs the item's tile + the CTA's rank)
-__device__ __forceinline__ SrcBox src_box(const TcParams &P, const TcItem &w, int bz, int e) {
-  const int c = w.parity;
-  const int cx = (c >> 2) & 1, cy = (c >> 1) & 1, cz = c & 1;
-  const int dx = P.off[c][e][0], dy = P.off[c][e][1], dz = P.off[c][e][2];
-  SrcBox b;
-  b.sp = (((cx + dx) & 1) << 2) | (((cy + dy) & 1) << 1) | ((cz + dz) & 1);
-  b.ox = w.bx * TILE_X + ((cx + dx) >> 1);
-  b.oy = w.by * TILE_Y + ((cy + dy) >> 1);
-  b.oz = bz * TILE_Z + ((cz + dz) >> 1);
-  b.slot = P.slot[c][e];
-  return b;
-}
-__device__ __forceinline__ long long tile_id(const TcParams &P, int level, int parity, int bx, int by, int bz) {
+// Every warp role skips the transfer vectors whose source box is empty (those A tiles are all zero) and the items whose
+// target tile is empty, so that sparse trees (surface or clustered distributions) cost only their occupied tiles.
+template <class PT>
+__device__ __forceinline__ long long tile_id(const PT &P, int level, int parity, int bx, int by, int bz) {
   const TcLevel &L = P.lv[level];
   const int TX = L.HX / TILE_X, TY = L.HY / TILE_Y, TZ = L.HZ / TILE_Z;
   return L.tile0 + (((long long)parity * TZ + bz) * TY + by) * TX + bx;
@@ -428,8 +420,8 @@ struct BusyMask {
   __device__ __forceinline__ bool src(int e) const { return (word(e >> 5) >> (e & 31)) & 1u; }
 };
 // G: the launch may hold compacted blocks (kernels without them compile the tile form alone)
-template <bool G = true>
-__device__ __forceinline__ BusyMask busy_mask(const TcParams &P, const TcItem &w) {
+template <bool G = true, class PT>
+__device__ __forceinline__ BusyMask busy_mask(const PT &P, const TcItem &w) {
   const unsigned *m = (G && w.blk >= 0) ? P.cbusy + 6LL * (P.lv[w.level].cb0 + w.blk)
                                  : P.busy + 6 * tile_id(P, w.level, w.parity, w.bx, w.by, w.bz);
   BusyMask b;
@@ -441,8 +433,8 @@ __device__ __forceinline__ BusyMask busy_mask(const TcParams &P, const TcItem &w
 // a transfer vector (or the item) only when it is idle for both tiles.  A level with an odd number of z tiles
 // has no tile bz + 1 in its last pair; that tile's A boxes lie outside the grid (zero-filled loads) and its
 // rows map to no cell.
-template <bool G = true>
-__device__ __forceinline__ BusyMask busy_mask_pair(const TcParams &P, const TcItem &w) {
+template <bool G = true, class PT>
+__device__ __forceinline__ BusyMask busy_mask_pair(const PT &P, const TcItem &w) {
   BusyMask b = busy_mask<G>(P, w);
   if (G && w.blk >= 0) {
     // compacted blocks come in pairs of one parity: block blk + 1 always exists (possibly without cells)
@@ -457,8 +449,8 @@ __device__ __forceinline__ BusyMask busy_mask_pair(const TcParams &P, const TcIt
   return b;
 }
 
-template <bool G = true>
-__device__ __forceinline__ TcItem decode_unit(const TcParams &P, int u) {
+template <bool G = true, class PT>
+__device__ __forceinline__ TcItem decode_unit(const PT &P, int u) {
   int level = P.l1;
   while (level > P.l0 && u >= P.lv[level].unit0 + P.lv[level].nunits) --level;
   const TcLevel &L = P.lv[level];
@@ -1563,23 +1555,19 @@ __device__ __forceinline__ int level_of(const long long *start, int l0, int l1, 
   return l;
 }
 
-__global__ void occ_mark_kernel(const __grid_constant__ TcParams P, const __grid_constant__ LevelCells C) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (g >= C.start[C.l1 + 1]) return;
+// a cell's mark, one up and right of its position in its parity's table
+__device__ __forceinline__ int *sat_mark(const TcTree &P, const LevelCells &C, long long g) {
   const int l = level_of(C.start, C.l0, C.l1, g);
   const TcLevel &L = P.lv[l];
   int ix, iy, iz;
   morton_decode3(C.keys[l][g - C.start[l]], ix, iy, iz);
   const int c = ((ix & 1) << 2) | ((iy & 1) << 1) | (iz & 1);
   const size_t SX = L.HX + 1, SY = L.HY + 1, SZ = L.HZ + 1;
-  int *sat = const_cast<int *>(L.sat);
-  sat[(((size_t)c * SZ + (iz >> 1) + 1) * SY + (iy >> 1) + 1) * SX + (ix >> 1) + 1] = 1;
+  return const_cast<int *>(L.sat) + (((size_t)c * SZ + (iz >> 1) + 1) * SY + (iy >> 1) + 1) * SX + (ix >> 1) + 1;
 }
-
-__global__ void sat_pass_kernel(const __grid_constant__ TcParams P, const __grid_constant__ LevelCells C, int axis) {
+// running sums along line g of an axis
+__device__ __forceinline__ void sat_line(const TcTree &P, const LevelCells &C, int axis, long long g) {
   const long long *ls = C.lines[axis];
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (g >= ls[C.l1 + 1]) return;
   const int l = level_of(ls, C.l0, C.l1, g);
   const long long t = g - ls[l];
   const TcLevel &L = P.lv[l];
@@ -1605,6 +1593,28 @@ __global__ void sat_pass_kernel(const __grid_constant__ TcParams P, const __grid
     sat[base + k * stride] = acc;
   }
 }
+__global__ void occ_mark_kernel(const __grid_constant__ TcTree P, const __grid_constant__ LevelCells C) {
+  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (g < C.start[C.l1 + 1]) *sat_mark(P, C, g) = 1;
+}
+__global__ void sat_pass_kernel(const __grid_constant__ TcTree P, const __grid_constant__ LevelCells C, int axis) {
+  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (g < C.lines[axis][C.l1 + 1]) sat_line(P, C, axis, g);
+}
+// The whole tables of a small tree (kSatSmall entries; height 5 has 7,600, height 6 47,000) by one CTA: the clear, the
+// marks and the three passes in one launch instead of five.
+constexpr long long kSatSmall = 16384;
+__global__ void __launch_bounds__(1024) sat_small_kernel(const __grid_constant__ TcTree P,
+                                                         const __grid_constant__ LevelCells C, int *__restrict__ sat,
+                                                         int n) {
+  for (int i = threadIdx.x; i < n; i += 1024) sat[i] = 0;
+  __syncthreads();
+  for (long long g = threadIdx.x; g < C.start[C.l1 + 1]; g += 1024) *sat_mark(P, C, g) = 1;
+  for (int axis = 0; axis < 3; ++axis) {
+    __syncthreads();
+    for (long long g = threadIdx.x; g < C.lines[axis][C.l1 + 1]; g += 1024) sat_line(P, C, axis, g);
+  }
+}
 
 // Whether a box of a parity grid holds a cell when its level is full (every cell of the level exists):
 // the parity grids then hold exactly the positions [0, side / 2) on each axis.
@@ -1613,38 +1623,39 @@ __device__ __forceinline__ bool box_nonempty_full(const TcLevel &L, int x0, int 
   return x0 < h && x0 + nx > 0 && y0 < h && y0 + ny > 0 && z0 < h && z0 + nz > 0;
 }
 
-// busy masks of every level: one thread per (tile, transfer vector); tiles are numbered across levels.  Bit l
-// of full_levels marks a full level, whose boxes are tested by their bounds instead of the summed-area
+// busy masks of every level: a warp per tile, lane e mod 32 for transfer vector e; tiles are numbered across levels.
+// Bit l of full_levels marks a full level, whose boxes are tested by their bounds instead of the summed-area
 // tables (which are then not built when every level is full).
-__global__ void busy_mask_kernel(const __grid_constant__ TcParams P, int l0, int l1, long long ntiles,
-                                 unsigned full_levels, unsigned *__restrict__ busy) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (g >= ntiles * 189) return;
-  const long long tg = g / 189;
-  const int e = (int)(g % 189);
-  int level = l0;
-  while (level < l1 && tg >= P.lv[level + 1].tile0) ++level;
+__global__ void __launch_bounds__(256) busy_mask_kernel(const __grid_constant__ TcTree P, long long ntiles,
+                                                        unsigned full_levels, unsigned *__restrict__ busy) {
+  const long long tg = (blockIdx.x * 256LL + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (tg >= ntiles) return;
+  int level = P.l0;
+  while (level < P.l1 && tg >= P.lv[level + 1].tile0) ++level;
   const TcLevel &L = P.lv[level];
   const long long tl = tg - L.tile0;
   const int TX = L.HX / TILE_X, TY = L.HY / TILE_Y, TZ = L.HZ / TILE_Z;
-  TcItem w;
-  w.level = (short)level;
-  w.blk = -1;
-  w.bx = (short)(tl % TX);
-  w.by = (short)((tl / TX) % TY);
-  w.bz = (short)((tl / ((long long)TX * TY)) % TZ);
-  w.parity = (short)(tl / ((long long)TX * TY * TZ));
-  unsigned *m = busy + 6 * tg;
-  const SrcBox b = src_box(P, w, w.bz, e);
+  const int x0 = (int)(tl % TX) * TILE_X, y0 = (int)((tl / TX) % TY) * TILE_Y,
+            z0 = (int)((tl / ((long long)TX * TY)) % TZ) * TILE_Z, c = (int)(tl / ((long long)TX * TY * TZ));
+  const int cx = (c >> 2) & 1, cy = (c >> 1) & 1, cz = c & 1;
   const bool full = (full_levels >> level) & 1u;
-  const bool src = full ? box_nonempty_full(L, b.ox, b.oy, b.oz, TILE_X, TILE_Y, TILE_Z)
-                        : box_count(L, b.sp, b.ox, b.oy, b.oz, TILE_X, TILE_Y, TILE_Z) > 0;
-  if (src) atomicOr(m + (e >> 5), 1u << (e & 31));
-  if (e == 0) {
-    const int x0 = w.bx * TILE_X, y0 = w.by * TILE_Y, z0 = w.bz * TILE_Z;
-    const bool tgt = full ? box_nonempty_full(L, x0, y0, z0, TILE_X, TILE_Y, TILE_Z)
-                          : box_count(L, w.parity, x0, y0, z0, TILE_X, TILE_Y, TILE_Z) > 0;
-    if (tgt) atomicOr(m + 5, 1u << 31);
+  // whether the box of parity grid p at (x, y, z) holds a cell
+  auto any = [&](int p, int x, int y, int z) {
+    return full ? box_nonempty_full(L, x, y, z, TILE_X, TILE_Y, TILE_Z)
+                : box_count(L, p, x, y, z, TILE_X, TILE_Y, TILE_Z) > 0;
+  };
+  for (int k = 0; k < 6; ++k) {
+    const int e = 32 * k + lane;
+    bool src = false;
+    if (e < 189) {
+      const int dx = cx + P.itab->off[c][e][0], dy = cy + P.itab->off[c][e][1], dz = cz + P.itab->off[c][e][2];
+      src = any(((dx & 1) << 2) | ((dy & 1) << 1) | (dz & 1), x0 + (dx >> 1), y0 + (dy >> 1), z0 + (dz >> 1));
+    } else if (e == 191) {
+      src = any(c, x0, y0, z0);  // bit 31 of word 5: the tile itself
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, src);
+    if (lane == 0) busy[6 * tg + k] = m;
   }
 }
 
@@ -1652,7 +1663,7 @@ __global__ void busy_mask_kernel(const __grid_constant__ TcParams P, int l0, int
 // the unit's target tile (either tile of a pair) is occupied, else 0.  Written to prefix[u], which the scan
 // below turns into exclusive prefix sums.
 // Whether a unit holds a target cell of the shard (cells [a, b) of its level in Morton order).
-__device__ bool unit_in_shard(const TcParams &P, const TcItem &w) {
+__device__ bool unit_in_shard(const TcTree &P, const TcItem &w) {
   const long long a = P.shard[2 + 2 * w.level], b = P.shard[3 + 2 * w.level];
   if (a >= b) return false;
   const TcLevel &L = P.lv[w.level];
@@ -1679,9 +1690,7 @@ __device__ bool unit_in_shard(const TcParams &P, const TcItem &w) {
   return false;
 }
 
-__global__ void unit_work_kernel(const __grid_constant__ TcParams P, int nunits, int *__restrict__ prefix) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nunits) return;
+__device__ __forceinline__ int unit_work(const TcTree &P, int u) {
   const TcItem w = decode_unit(P, u);
   const BusyMask b = P.pair ? busy_mask_pair(P, w) : busy_mask(P, w);
   int n = 0;
@@ -1690,17 +1699,27 @@ __global__ void unit_work_kernel(const __grid_constant__ TcParams P, int nunits,
     for (int k = 0; k < 5; ++k) n += __popc(b.w[k]);
     n += __popc(b.w[5] & ((1u << (189 - 160)) - 1u));
   }
-  prefix[u] = n;
+  return n;
+}
+__global__ void unit_work_kernel(const __grid_constant__ TcTree P, int nunits, int *__restrict__ prefix) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u < nunits) prefix[u] = unit_work(P, u);
 }
 
-// In-place exclusive prefix sums of prefix[0, n) with the total in prefix[n] (one block of 1024 threads).
-__global__ void __launch_bounds__(1024) unit_scan_kernel(int n, int *__restrict__ prefix) {
+// In-place exclusive prefix sums of prefix[0, n) with the total in prefix[n] (one block of 1024 threads).  WORK: of
+// at most 1024 units, whose work the threads take themselves.
+template <bool WORK>
+__global__ void __launch_bounds__(1024) unit_scan_kernel(const __grid_constant__ TcTree P, int n,
+                                                         int *__restrict__ prefix) {
   __shared__ int part[1024];
   const int t = threadIdx.x;
   const int chunk = (n + 1023) / 1024;
   const int a = min(n, t * chunk), b = min(n, a + chunk);
   int sum = 0;
-  for (int i = a; i < b; ++i) sum += prefix[i];
+  if (WORK)
+    sum = t < n ? unit_work(P, t) : 0;
+  else
+    for (int i = a; i < b; ++i) sum += prefix[i];
   part[t] = sum;
   __syncthreads();
   for (int off = 1; off < 1024; off <<= 1) {
@@ -1710,10 +1729,14 @@ __global__ void __launch_bounds__(1024) unit_scan_kernel(int n, int *__restrict_
     __syncthreads();
   }
   int run = part[t] - sum;  // exclusive start of this thread's chunk
-  for (int i = a; i < b; ++i) {
-    const int v = prefix[i];
-    prefix[i] = run;
-    run += v;
+  if (WORK) {
+    if (t < n) prefix[t] = run;
+  } else {
+    for (int i = a; i < b; ++i) {
+      const int v = prefix[i];
+      prefix[i] = run;
+      run += v;
+    }
   }
   if (t == 1023) prefix[n] = part[1023];
 }
@@ -1891,7 +1914,8 @@ struct CBlocks {
   int l0, l1;
   int b0[kMaxHeight + 1];  // first block of each level; levels that are not compacted have none
 };
-__global__ void __launch_bounds__(128) cbusy_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CBlocks B,
+// Four groups of 128 threads share the transfer vectors.
+__global__ void __launch_bounds__(512) cbusy_kernel(const __grid_constant__ TcTree P, const __grid_constant__ CBlocks B,
                                                     unsigned *__restrict__ cbusy) {
   __shared__ unsigned m[6];
   const int gb = blockIdx.x;
@@ -1901,7 +1925,7 @@ __global__ void __launch_bounds__(128) cbusy_kernel(const __grid_constant__ TcPa
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 6) m[threadIdx.x] = 0;
   __syncthreads();
-  const int code = L.crow[(long long)(gb - B.b0[l]) * 128 + threadIdx.x];
+  const int code = L.crow[(long long)(gb - B.b0[l]) * 128 + (threadIdx.x & 127)];
   int gx = 0, gy = 0, gz = 0, par = 0;
   if (code >= 0) {
     par = code >> 28;
@@ -1914,10 +1938,11 @@ __global__ void __launch_bounds__(128) cbusy_kernel(const __grid_constant__ TcPa
   const unsigned any = __ballot_sync(0xffffffffu, code >= 0);
   // every row of a block has the same parity; rows without a cell take the first valid row's
   par = __shfl_sync(0xffffffffu, par, any ? __ffs(any) - 1 : 0);
-  for (int e = 0; e < 189; ++e) {
+#pragma unroll 4
+  for (int e = threadIdx.x >> 7; e < 189; e += 4) {
     bool occ = false;
     if (code >= 0) {
-      const int sx = gx + P.off[par][e][0], sy = gy + P.off[par][e][1], sz = gz + P.off[par][e][2];
+      const int sx = gx + P.itab->off[par][e][0], sy = gy + P.itab->off[par][e][1], sz = gz + P.itab->off[par][e][2];
       occ = sx >= 0 && sx < L.side && sy >= 0 && sy < L.side && sz >= 0 && sz < L.side &&
             L.grid[((long long)sz * L.side + sy) * L.side + sx] >= 0;
     }
@@ -2283,7 +2308,6 @@ b200fmm_status tc_init(Context &c) {
   t->params = new TcParams();
   std::memset(t->params, 0, sizeof(TcParams));
   std::memcpy(t->params->off, c.itab.off, sizeof(t->params->off));
-  std::memcpy(t->params->slot, c.itab.slot, sizeof(t->params->slot));
   // symmetric Chebyshev operators run in their compressed (low-rank) form; B200FMM_TC_LOWRANK=0 keeps the
   // dense operators
   bool lr = c.cfg.kernel == B200FMM_CHEB_SYM && !c.sym_ranks.empty();
@@ -2613,11 +2637,23 @@ static b200fmm_status tc_prepare(Context &c) {
   // a group of two chunks holds two stages while the producer fills the next ones: only with 5 or more
   if (const char *e = getenv("B200FMM_TC_SEGMENTS")) P.nseg = std::max(1, std::min(t->NK, atoi(e)));
   std::memcpy(P.off, c.itab.off, sizeof(P.off));
-  std::memcpy(P.slot, c.itab.slot, sizeof(P.slot));
   P.status = c.d_status;
   t->built_for_N = c.N;
   t->built_for_gen = c.tree_gen;
   return B200FMM_OK;
+}
+
+static TcTree tree_params(const Context &c, const TcParams &P) {
+  TcTree T{};
+  std::memcpy(T.lv, P.lv, sizeof(T.lv));
+  T.itab = c.d_itab;
+  T.busy = P.busy;
+  T.cbusy = P.cbusy;
+  T.l0 = 2;
+  T.l1 = c.H - 1;
+  T.pair = P.pair;
+  T.shard = P.shard;
+  return T;
 }
 
 // Per tree: which sparse levels run compacted, and their cells grouped by parity into 128-row blocks.
@@ -2842,7 +2878,7 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
       t.cbusy_cap = nb_all;
     }
     P.cbusy = t.cbusy;
-    cbusy_kernel<<<nb_all, 128, 0, c.stream>>>(P, B, t.cbusy);
+    cbusy_kernel<<<nb_all, 512, 0, c.stream>>>(tree_params(c, P), B, t.cbusy);
     ++c.launches;
   }
   return B200FMM_OK;
@@ -2870,15 +2906,17 @@ b200fmm_status tc_tree_setup(Context &c) {
       C.lines[1][l + 1] = C.lines[1][l] + 8 * (HZ + 1) * (HX + 1);
       C.lines[2][l + 1] = C.lines[2][l] + 8 * (HY + 1) * (HX + 1);
     }
-    const TcParams &P0 = *t->params;
+    const TcTree P0 = tree_params(c, *t->params);
     // full levels (every cell present, as in uniform trees) need no occupancy tables
     unsigned full_levels = 0;
     for (int l = 2; l <= LL; ++l)
       if (c.lv[l].n == (1LL << (3 * l))) full_levels |= 1u << l;
     const bool all_full = full_levels == (((1u << (LL + 1)) - 1u) & ~3u);
     if (t->lr) t->yparams->full_levels = full_levels;
-    B200_CUDA(cudaMemsetAsync(t->busy, 0, sizeof(unsigned) * 6 * t->ntiles_all, c.stream));
-    if (!all_full) {
+    if (!all_full && t->satn <= kSatSmall) {
+      sat_small_kernel<<<1, 1024, 0, c.stream>>>(P0, C, t->sat, (int)t->satn);
+      ++c.launches;
+    } else if (!all_full) {
       B200_CUDA(cudaMemsetAsync(t->sat, 0, t->satn * sizeof(int), c.stream));
       if (C.start[LL + 1] > 0) {
         occ_mark_kernel<<<grid_for(C.start[LL + 1], 256), 256, 0, c.stream>>>(P0, C);
@@ -2889,20 +2927,23 @@ b200fmm_status tc_tree_setup(Context &c) {
         ++c.launches;
       }
     }
-    busy_mask_kernel<<<grid_for(t->ntiles_all * 189, 256), 256, 0, c.stream>>>(P0, 2, LL, t->ntiles_all, full_levels,
-                                                                                 t->busy);
+    busy_mask_kernel<<<grid_for(t->ntiles_all * 32, 256), 256, 0, c.stream>>>(P0, t->ntiles_all, full_levels, t->busy);
     ++c.launches;
     // compacted levels: placement, unit numbering and block masks
     B200_CHECK(compact_setup(c, *t));
     // the work of every unit of every level and its prefix sums, from which each launch splits its units
     // into ranges of equal work
     t->params->shard = c.shard_count > 1 ? c.d_shard : nullptr;
-    TcParams Pw = *t->params;
-    Pw.l0 = 2;
-    Pw.l1 = LL;
-    unit_work_kernel<<<grid_for(t->nunits_all, 256), 256, 0, c.stream>>>(Pw, t->nunits_all, t->prefix);
-    unit_scan_kernel<<<1, 1024, 0, c.stream>>>(t->nunits_all, t->prefix);
-    c.launches += 2;
+    const TcTree Pw = tree_params(c, *t->params);
+    if (t->nunits_all <= 1024) {
+      unit_scan_kernel<true><<<1, 1024, 0, c.stream>>>(Pw, t->nunits_all, t->prefix);
+    } else {
+      unit_work_kernel<<<grid_for(t->nunits_all, 256), 256, 0, c.stream>>>(Pw, t->nunits_all, t->prefix);
+      unit_scan_kernel<false><<<1, 1024, 0, c.stream>>>(Pw, t->nunits_all, t->prefix);
+      ++c.launches;
+    }
+    ++c.launches;
+    B200_CUDA(cudaGetLastError());
     t->sat_serial = c.tree_serial;
   }
   return B200FMM_OK;
