@@ -36,7 +36,7 @@
 // two to 1e-12 relative.
 //
 // Measured, all levels, before (DFMA tiles of 128 x 128, one launch per level and phase; dense: one CTA per target
-// cell) and after: 1M uniform, order 7, height 6: 23.1 -> 9.4 ms (phase 1 26 TFLOP/s of operator work; phase 2, with
+// cell) and after: 1M uniform, order 7, height 6: 23.1 -> 9.25 ms (phase 1 26 TFLOP/s of operator work; phase 2, with
 // the missing sources at the box faces and the padding counted, 31); 20,000 points, order 7, height 5: 6.2 -> 1.4 ms;
 // 65,537 points, dense order 5, height 5: 7.6 -> 0.94 ms; 500,009 points on a surface, Lagrange order 6, height 7:
 // 19.1 -> 1.7 ms by pairs (7.0 ms by target tiles: 64 neighbouring targets of a surface share 4.1 times the sources
@@ -64,7 +64,7 @@ __host__ __device__ constexpr int g_mb(int p) {
 struct Sym64 {
   bool dense = false;
   int lda = 0;                       // row length of the phase-2 operators: p^3 rounded up to 8
-  int ysum[8] = {0};                 // rows of Vs_sp: the ranks of the slots parity sp feeds, each rounded up to 4
+  int ysum[8] = {0};                 // rows of Vs_sp: the ranks of the slots parity sp feeds, each rounded up to 2
   int yrank[8] = {0};                // the same without the rounding (the algorithmic count)
   int ldv[8] = {0};                  // row length of Vs_sp: ysum rounded up to 8
   long long vs_off[8] = {0};         // element offset of Vs_sp in d_vs
@@ -627,6 +627,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) gemm64_kernel(const __grid_const
       cp_commit();
     sources(st0 + u + 1);
   }
+  const bool own = wn * 16 < ntile;  // Y, PAIRS: the tile has cells of this warp's
   const int ar = (lane & 3) * LDA + wm * MB * 8 + (lane >> 2);
   const int br = (wn * 16 + (lane >> 2)) * G_LDB + (lane & 3);
   for (int st = st0; st < st1; ++st) {
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(G_THREADS, 2) gemm64_kernel(const __grid_const
       const int q = st * 4 + g;
       if (q >= groups) break;
       unsigned m = 3u;
+      if (MODE != G_TILES && !own) break;
       if (MODE == G_TILES) {
         int ei, gi;
         locate(q, ei, gi);
@@ -794,8 +796,8 @@ b200fmm_status sym64_prepare(Context &c, const double *d_Ut, const double *d_Vt,
   const int nn = c.nn;
   s->lda = (nn + 7) & ~7;
   // the slots each source parity feeds: entry e of child type ct reads the cell at offset itab.off[ct][e], whose
-  // parity is ct's parity plus that offset, per axis.  Each slot's rows of Y start at a multiple of 4, so that a K
-  // group never crosses slots and 16-byte copies are aligned.
+  // parity is ct's parity plus that offset, per axis.  Each slot's rows of Y start at a multiple of 2, so that 16-byte
+  // copies are aligned.
   std::vector<int> ybase(8 * 343, -1);
   std::vector<int3> vrows;
   std::vector<long long> vfirst(8);
@@ -810,7 +812,7 @@ b200fmm_status sym64_prepare(Context &c, const double *d_Ut, const double *d_Vt,
       if (fed[t]) {
         if (toff[t] < 0) return fail(B200FMM_ERR_INVALID, "symmetric operators: a far slot has no factor");
         ybase[sp * 343 + t] = (int)(vrows.size() - vfirst[sp]);
-        for (int q = 0; q < ((trank[t] + 3) & ~3); ++q)
+        for (int q = 0; q < ((trank[t] + 1) & ~1); ++q)
           vrows.push_back(q < trank[t] ? make_int3((int)toff[t], trank[t], q) : make_int3(0, 0, 0));
         s->yrank[sp] += trank[t];
       }
