@@ -262,7 +262,7 @@ __device__ __forceinline__ void two_sum(float &hi, float &lo, float v) {
   lo += err;
 }
 
-constexpr int P2P32_WARPS = 4;   // target leaves per CTA (one warp each)
+constexpr int P2P32_WARPS = 2;   // work items per CTA (one warp each): few, so that a long one holds little else up
 constexpr int P2P32_STAGE = 56;  // source records (112 particles) per bulk-copy stage
 constexpr int P2P32_FLUSH = 24;  // records per lane whose sums enter the compensated sums together
 constexpr int P2P32_TGT = 2;     // targets per lane
@@ -353,8 +353,8 @@ __device__ __forceinline__ void p2p_record(const float4 *__restrict__ s, int k, 
 // sum per stage, about half of the issued instructions were not the pairs'.  Two targets alone changed nothing; with
 // stages of 56 records (the three z-neighbours of a leaf of 30 are one stage), packed compensated sums of both targets
 // after every 24 records of a lane (chains no longer than before: the error is 0.9-1.0 of the earlier kernel's) and
-// 126 registers (4 CTAs per SM): 1M uniform 0.885 -> 0.82 ms, 2M on a surface 6.13 -> 5.5 ms, 200k in leaves of 49
-// 0.345 -> 0.28 ms.  Sums after every 16 records cost 4 % more, after every 64 give 2 % but a larger error.
+// 128 registers: 1M uniform 0.885 -> 0.81 ms, 2M on a surface 6.13 -> 5.68 ms, 200k in leaves of 49 0.347 -> 0.285
+// ms.  (Five CTAs of four warps at 100 registers and stages of 44: 0.95, 5.98 and 0.31 ms.)  Sums after every 16 records cost 4 % more, after every 64 give 2 % but a larger error.
 // The targets are taken 64, 32, 16 or 8 at a time (p2p_chunk); 32 (16, 8) targets occupy 16 (8, 4) lanes and are
 // replicated over 2 (4, 8) lane groups, each group walking every 2nd (4th, 8th) source record, and the groups' sums
 // are combined by shuffles at the end, so that small and ragged leaves keep the lanes busy.
@@ -400,7 +400,7 @@ __device__ __forceinline__ bool p2p_item(long long item, long long nleaves, cons
 // slots in use, and 33..48 as 32 and the rest.
 __device__ __forceinline__ int p2p_chunk(long long left) { return left > 48 ? 64 : left > 16 ? 32 : left > 8 ? 16 : 8; }
 
-__global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_kernel(
+__global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
     const long long *__restrict__ chunk_base, int whole, int isize, const long long *__restrict__ shard,
@@ -682,8 +682,8 @@ __device__ __forceinline__ void p2p_record_mrhs(const float4 *__restrict__ s, in
 // One warp per work item and group of MR_G right-hand sides (grid.y): runs of records in bulk-copy stages, one target
 // per lane (two would need 64 accumulator registers more), lane groups for small leaves, per-stage two-sums.  With
 // the groups one after the other in a warp, 4,096 leaves of 61 gave 1.7 waves of long items: 3.7 -> 2.6 ms with the
-// groups on the grid, items of 32 targets and the longer stages (250k points x 16).
-__global__ void __launch_bounds__(P2P32_WARPS * 32, 4) p2p_fp32_mrhs_kernel(
+// groups on the grid, items of 32 targets and the longer stages (250k points x 16).  Two warps per CTA.
+__global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
     const long long *__restrict__ chunk_base, int whole, int isize, const long long *__restrict__ shard,
