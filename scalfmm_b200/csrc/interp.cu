@@ -97,14 +97,15 @@ __device__ __forceinline__ void record_max(unsigned long long *slots, double mx)
 // M[nx,ny,nz] = sum_j q_j Sx_j[nx] Sy_j[ny] Sz_j[nz].  The threads first evaluate the 1-D weights of up to 64
 // particles (one each) into shared memory; then thread t < p^2 owns the node line (ny, nz) = (t % p, t / p)
 // and keeps its p sums over nx in registers: per particle one product q Sy Sz and p FMAs with the
-// broadcast Sx row, instead of three shared-memory reads per node and particle.  Several right-hand sides share the
-// weights of a leaf of one chunk.  (Measured slower, 1M uniform, order 7, height 6: 128 threads, the weights along
+// broadcast Sx row, instead of three shared-memory reads per node and particle.  Several right-hand sides are taken
+// two at a time, with the weights of a leaf of one chunk evaluated once (250k points x 16, order 7: 0.48 -> 0.29
+// ms: the shared-memory reads of the weights bound it).  (Measured slower, 1M uniform, order 7, height 6: 128 threads, the weights along
 // rows of particles, two particles per load and two node lines per lane, 0.250 against 0.148 ms: 96 registers with
 // spills and three more barriers per leaf cost more than the halved shared-memory reads give.)
 constexpr int P2M_THREADS = 64;
-constexpr int L2P_WARPS = 2;  // L2P: leaves per CTA, one warp each (static shared memory <= 48 KB at order 8)
+constexpr int L2P_WARPS = 1;  // L2P: leaves per CTA, one warp each (static shared memory <= 48 KB at order 8)
 
-template <int P, bool LAGR>
+template <int P, bool LAGR, int NR>
 __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ keys,
     const long long *__restrict__ leaf_start, const double *__restrict__ x, const double *__restrict__ y,
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
     double *__restrict__ M, unsigned long long *__restrict__ mmax) {
   constexpr int p = P, nn = P * P * P, PX = P <= 6 ? (P + 1) & ~1 : 10;  // Sx rows: 16-byte steps, spread over the banks
   __shared__ __align__(16) double Wx[P2M_THREADS][PX];
-  __shared__ double Wy[P2M_THREADS][P], Wz[P2M_THREADS][P], Q[P2M_THREADS];
+  __shared__ double Wy[P2M_THREADS][P], Wz[P2M_THREADS][P], Q[NR][P2M_THREADS];
   const int t = threadIdx.x;
   const long long leaf = blockIdx.x;
   int ix, iy, iz;
@@ -121,18 +122,20 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
   const long long s0 = leaf_start[leaf], s1 = leaf_start[leaf + 1];
   const int ny = t % p, nz = t / p;
   const bool owner = t < p * p;
-  for (int r = 0; r < R; ++r) {
-    double acc[P];
+  for (int r0 = 0; r0 < R; r0 += NR) {
+    double acc[NR][P];
 #pragma unroll
-    for (int k = 0; k < p; ++k) acc[k] = 0.0;
+    for (int u = 0; u < NR; ++u)
+#pragma unroll
+      for (int k = 0; k < p; ++k) acc[u][k] = 0.0;
     for (long long b = s0; b < s1; b += P2M_THREADS) {
       const int cnt = (int)min((long long)P2M_THREADS, s1 - b);
       __syncthreads();
       if (t < cnt) {
         const long long i = b + t;
-        const double pos[3] = {x[i], y[i], z[i]};
-        double wv[P];
-        if (r == 0 || s1 - s0 > P2M_THREADS) {
+        if (r0 == 0 || s1 - s0 > P2M_THREADS) {
+          const double pos[3] = {x[i], y[i], z[i]};
+          double wv[P];
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             const double a = ctr[d] - leaf_w / 2, bb = ctr[d] + leaf_w / 2;
@@ -142,25 +145,34 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
             for (int k = 0; k < p; ++k) dst[k] = wv[k];
           }
         }
-        Q[t] = q[(long long)r * N + i];
+#pragma unroll
+        for (int u = 0; u < NR; ++u) Q[u][t] = r0 + u < R ? q[(long long)(r0 + u) * N + i] : 0.0;
       }
       __syncthreads();
       if (owner) {
         for (int j = 0; j < cnt; ++j) {
-          const double w = Q[j] * Wy[j][ny] * Wz[j][nz];
+          const double wyz = Wy[j][ny] * Wz[j][nz];
 #pragma unroll
-          for (int k = 0; k < p; ++k) acc[k] += w * Wx[j][k];
+          for (int u = 0; u < NR; ++u) {
+            const double w = Q[u][j] * wyz;
+#pragma unroll
+            for (int k = 0; k < p; ++k) acc[u][k] += w * Wx[j][k];
+          }
         }
       }
     }
     double mx = 0.0;
     if (owner) {
-      double *out = M + (leaf * R + r) * nn + (nz * p + ny) * p;
 #pragma unroll
-      for (int k = 0; k < p; ++k) {
-        const double v = out[k] + acc[k];
-        out[k] = v;
-        mx = fmax(mx, fabs(v));
+      for (int u = 0; u < NR; ++u) {
+        if (r0 + u >= R) break;
+        double *out = M + (leaf * R + r0 + u) * nn + (nz * p + ny) * p;
+#pragma unroll
+        for (int k = 0; k < p; ++k) {
+          const double v = out[k] + acc[u][k];
+          out[k] = v;
+          mx = fmax(mx, fabs(v));
+        }
       }
     }
     if (mmax) record_max(mmax, mx);
@@ -332,6 +344,10 @@ __device__ __forceinline__ void copy_block(double *dst, const double *__restrict
 // The leaf's local expansion sits in shared memory; each lane contracts it with its particle's weights one
 // axis at a time: the x weights in registers, the y and z weights (and derivatives) in the lane's own
 // shared-memory row, so that the loops over y and z need no register indexing and the kernel stays small.
+// One warp per CTA, so that a leaf that ends frees its place at once, and all lanes through the last round together: 1M
+// points, order 7, height 6 0.206 -> 0.184 ms, 2M on a surface 0.368 -> 0.348 ms, 200k clustered 0.139 -> 0.115 ms (two
+// warps per CTA, lanes leaving one by one before).  Capping the registers for more CTAs, or two right-hand sides at a
+// time, was slower.
 template <int P, bool LAGR>
 __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ keys,
@@ -354,28 +370,33 @@ __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
   const double cx = cx0 + (ix + 0.5) * leaf_w, cy = cy0 + (iy + 0.5) * leaf_w, cz = cz0 + (iz + 0.5) * leaf_w;
   const double jac = 2.0 / leaf_w;
   const long long s0 = leaf_start[leaf], s1 = leaf_start[leaf + 1];
-  for (int r = 0; r < R; ++r) {
-    __syncwarp();
-    copy_block<nn, 32>(Lw, L + (leaf * R + r) * nn, lane);
-    __syncwarp();
-    for (long long i = s0 + lane; i < s1; i += 32) {
-      double wx[P], dwx[P];
-      {
-        double t[P], dt[P];
-        basis_eval<P, LAGR>((2.0 * y[i] - 2.0 * cy) / leaf_w, t, dt);
+  for (long long i0 = s0; i0 < s1; i0 += 32) {
+    // every lane goes through a last partial round (a leaf's first particle where there is none)
+    const bool on = i0 + lane < s1;
+    const long long i = on ? i0 + lane : s0;
+    double wx[P], dwx[P];
+    {
+      double t[P], dt[P];
+      basis_eval<P, LAGR>((2.0 * y[i] - 2.0 * cy) / leaf_w, t, dt);
 #pragma unroll
-        for (int k = 0; k < p; ++k) {
-          wy[k] = t[k];
-          dwy[k] = dt[k];
-        }
-        basis_eval<P, LAGR>((2.0 * z[i] - 2.0 * cz) / leaf_w, t, dt);
-#pragma unroll
-        for (int k = 0; k < p; ++k) {
-          wz[k] = t[k];
-          dwz[k] = dt[k];
-        }
+      for (int k = 0; k < p; ++k) {
+        wy[k] = t[k];
+        dwy[k] = dt[k];
       }
-      basis_eval<P, LAGR>((2.0 * x[i] - 2.0 * cx) / leaf_w, wx, dwx);
+      basis_eval<P, LAGR>((2.0 * z[i] - 2.0 * cz) / leaf_w, t, dt);
+#pragma unroll
+      for (int k = 0; k < p; ++k) {
+        wz[k] = t[k];
+        dwz[k] = dt[k];
+      }
+    }
+    basis_eval<P, LAGR>((2.0 * x[i] - 2.0 * cx) / leaf_w, wx, dwx);
+    for (int r = 0; r < R; ++r) {
+      if (i0 == s0 || R > 1) {
+        __syncwarp();
+        copy_block<nn, 32>(Lw, L + (leaf * R + r) * nn, lane);
+        __syncwarp();
+      }
       double pv = 0, gx = 0, gy = 0, gz = 0;
 #pragma unroll 1
       for (int kz = 0; kz < p; ++kz) {
@@ -401,12 +422,14 @@ __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
         gy += zk * bzy;
         gz += dwz[kz] * bz;
       }
-      const long long j = (long long)r * N + i;
-      const double qq = q[j];
-      phi[j] += pv;
-      fx[j] += gx * jac * qq;
-      fy[j] += gy * jac * qq;
-      fz[j] += gz * jac * qq;
+      if (on) {
+        const long long j = (long long)r * N + i;
+        const double qq = q[j];
+        phi[j] += pv;
+        fx[j] += gx * jac * qq;
+        fy[j] += gy * jac * qq;
+        fz[j] += gz * jac * qq;
+      }
     }
   }
 }
@@ -438,14 +461,13 @@ b200fmm_status run_p2m(Context &c) {
   const bool lagr = c.cfg.kernel == B200FMM_LAGRANGE;
   unsigned long long *mmax = c.mmax_out ? c.mmax_out + (size_t)LL * kMmaxSlots : nullptr;
 #define B200_P2M(PV)                                                                                        \
-  case PV:                                                                                                  \
-    if (lagr)                                                                                               \
-      p2m_kernel<PV, true><<<(unsigned)L.n, P2M_THREADS, 0, c.stream>>>(                                     \
-          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.M, mmax);              \
-    else                                                                                                    \
-      p2m_kernel<PV, false><<<(unsigned)L.n, P2M_THREADS, 0, c.stream>>>(                                    \
-          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.M, mmax);              \
-    break;
+  case PV: {                                                                                                \
+    auto kernel = lagr ? (c.R > 1 ? p2m_kernel<PV, true, 2> : p2m_kernel<PV, true, 1>)                      \
+                       : (c.R > 1 ? p2m_kernel<PV, false, 2> : p2m_kernel<PV, false, 1>);                   \
+    kernel<<<(unsigned)L.n, P2M_THREADS, 0, c.stream>>>(c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, \
+                                                        c.d_q, x0, y0, z0, lw, L.M, mmax);                  \
+    break;                                                                                                  \
+  }
   switch (c.p) {
     B200_P2M(3) B200_P2M(4) B200_P2M(5) B200_P2M(6) B200_P2M(7) B200_P2M(8)
     default: return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
