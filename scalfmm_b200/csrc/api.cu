@@ -32,16 +32,43 @@ b200fmm_status ensure_scratch(Context &c, size_t bytes) {
   return B200FMM_OK;
 }
 
-b200fmm_status check_status(Context &c) {
-  int st[4] = {0, 0, 0, 0};
-  B200_CUDA(cudaMemcpyAsync(st, c.d_status, sizeof(st), cudaMemcpyDeviceToHost, c.stream));
-  B200_CUDA(cudaStreamSynchronize(c.stream));
+b200fmm_status ensure_stage(Context &c, size_t bytes) {
+  if (c.h_stage_bytes >= bytes) return B200FMM_OK;
+  if (c.h_stage) cudaFreeHost(c.h_stage);
+  c.h_stage = nullptr;
+  c.h_stage_bytes = 0;
+  size_t cap = 64 << 10;
+  while (cap < bytes) cap *= 2;
+  if (cudaMallocHost(&c.h_stage, cap) != cudaSuccess) {
+    cudaGetLastError();  // the caller copies the arrays one by one
+    c.h_stage = nullptr;
+    return B200FMM_ERR_OOM;
+  }
+  c.h_stage_bytes = cap;
+  return B200FMM_OK;
+}
+
+// The status words' copy is queued behind the work that it reports; read_status() looks at it after a wait.
+static int *status_words(Context &c) { return (int *)((char *)c.h_pinned + kPinnedCounts); }
+static b200fmm_status queue_status(Context &c) {
+  if (!c.h_pinned) return B200FMM_OK;  // no particles yet, so no kernel that could have set a word
+  B200_CUDA(cudaMemcpyAsync(status_words(c), c.d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  return B200FMM_OK;
+}
+static b200fmm_status read_status(Context &c) {
+  if (!c.h_pinned) return B200FMM_OK;
+  const int *st = status_words(c);
   if (st[0] || st[1] || st[2] || st[3]) {
-    cudaMemsetAsync(c.d_status, 0, sizeof(st), c.stream);
+    cudaMemsetAsync(c.d_status, 0, 4 * sizeof(int), c.stream);
     return fail(B200FMM_ERR_CUDA, std::string("a device wait ran out of its iteration budget (") +
                                       (st[0] ? "P2P" : st[1] ? "M2L" : "kernel") + ")");
   }
   return B200FMM_OK;
+}
+b200fmm_status check_status(Context &c) {
+  B200_CHECK(queue_status(c));
+  B200_CUDA(cudaStreamSynchronize(c.stream));
+  return read_status(c);
 }
 
 namespace {
@@ -145,6 +172,8 @@ void destroy_context(b200fmm_context *c) {
                   (void *)c->d_cls_slots, (void *)c->d_status, (void *)c->d_mmax, (void *)c->d_Ut, (void *)c->d_Vt,
                   (void *)c->d_toff, (void *)c->d_trank, c->d_scratch, (void *)c->d_out, (void *)c->d_shard})
     if (p) cudaFree(p);
+  if (c->h_pinned) cudaFreeHost(c->h_pinned);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->events_ready)
     for (auto &e : c->ev) cudaEventDestroy(e);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -648,10 +677,18 @@ b200fmm_status b200fmm_get_results(b200fmm_handle h, double *phi, double *fx, do
                                                               o + n * c.R, o + 2 * n * c.R, o + 3 * n * c.R);
   B200_CUDA(cudaGetLastError());
   double *dst[4] = {phi, fx, fy, fz};
-  for (int k = 0; k < 4; ++k)
-    if (dst[k]) B200_CUDA(cudaMemcpyAsync(dst[k], o + k * n * c.R, bytes, cudaMemcpyDeviceToHost, c.stream));
+  const bool staged = 4 * bytes <= kStageOut && ensure_stage(c, 4 * bytes) == B200FMM_OK;
+  if (staged)
+    B200_CUDA(cudaMemcpyAsync(c.h_stage, o, 4 * bytes, cudaMemcpyDeviceToHost, c.stream));
+  else
+    for (int k = 0; k < 4; ++k)
+      if (dst[k]) B200_CUDA(cudaMemcpyAsync(dst[k], o + k * n * c.R, bytes, cudaMemcpyDeviceToHost, c.stream));
+  B200_CHECK(queue_status(c));
   B200_CUDA(cudaStreamSynchronize(c.stream));
-  return check_status(c);
+  if (staged)
+    for (int k = 0; k < 4; ++k)
+      if (dst[k]) std::memcpy(dst[k], (char *)c.h_stage + k * bytes, bytes);
+  return read_status(c);
 }
 
 // Results to the host without waiting: staged in the caller's order on the handle's stream, then copied on a
@@ -711,9 +748,10 @@ b200fmm_status b200fmm_set_shard(b200fmm_handle h, int rank, int count) {
 b200fmm_status b200fmm_synchronize(b200fmm_handle h) {
   B200_CHECK(check_handle(h));
   B200_CHECK(set_device(*h));
+  B200_CHECK(queue_status(*h));
   B200_CUDA(cudaStreamSynchronize(h->stream));
   B200_CUDA(cudaStreamSynchronize(h->stream_out));
-  return check_status(*h);
+  return read_status(*h);
 }
 
 b200fmm_status b200fmm_tree_info(b200fmm_handle h, long long *ncells, long long *nparticles) {

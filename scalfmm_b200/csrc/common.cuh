@@ -163,7 +163,11 @@ struct Context {
   unsigned *d_cnt = nullptr;              // radix histograms
   double *d_stage = nullptr;              // host input staged on the device
   int *d_err = nullptr;                   // domain error flag; from byte 16 the cell count of each level
-  long long *h_pinned = nullptr;          // small pinned host buffer for counts
+  long long *h_pinned = nullptr;          // small pinned host buffer: counts of the tree build (kPinnedCounts), status
+  // pinned staging for small host inputs and results, one copy each way instead of one per array (grow-only, at most
+  // kStageOut bytes)
+  void *h_stage = nullptr;
+  size_t h_stage_bytes = 0;
   int tree_gen = 0;                       // bumped whenever a tree buffer moves
 
   // device status words set by kernels whose bounded waits ran out (0 = fine); checked by the host at
@@ -194,6 +198,13 @@ struct Context {
 
 b200fmm_status ensure_scratch(Context &c, size_t bytes);
 b200fmm_status check_status(Context &c);
+// Host arrays up to these sizes (all of a call's arrays together) go through the handle's pinned staging buffer.  A
+// copy from or to pageable memory costs the host 10-30 us whatever its size and waits for the device; one copy of
+// everything and a memcpy cost less up to here: results of 20,000 points 165 -> 85 us, inputs of 2,003 points 50 -> 25
+// us; inputs of 20,000 points cost the same either way.
+constexpr size_t kStageIn = 256 << 10, kStageOut = 4 << 20;
+b200fmm_status ensure_stage(Context &c, size_t bytes);
+constexpr size_t kPinnedCounts = sizeof(long long) * 64 + sizeof(int) * 344;
 
 // ---- module entry points -------------------------------------------------------------------------
 // precompute.cu

@@ -18,6 +18,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cstring>
 
 namespace b200 {
 
@@ -664,8 +665,6 @@ void free_tree(Context &c) {
   dfree(c.d_cnt);
   dfree(c.d_stage);
   dfree(c.d_err);
-  if (c.h_pinned) cudaFreeHost(c.h_pinned);
-  c.h_pinned = nullptr;
   for (int l = 0; l < kMaxHeight; ++l) {
     Level &L = c.lv[l];
     dfree(L.keys);
@@ -727,7 +726,7 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
   cudaStream_t s = c.stream;
   c.tree_launches = 0;
   c.packed32 = false;
-  if (!c.h_pinned) B200_CUDA(cudaMallocHost((void **)&c.h_pinned, sizeof(long long) * 64 + sizeof(int) * 344));
+  if (!c.h_pinned) B200_CUDA(cudaMallocHost((void **)&c.h_pinned, kPinnedCounts + 4 * sizeof(int)));
   // particle-sized buffers
   size_t cap;
   cap = c.cap_N;
@@ -771,13 +770,28 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
     // previous evaluation is still executing on the main stream.  The staging buffer is rewritten only after
     // its last main-stream reader (the previous build's gather, or set_charges' gather) has run.  The keys wait
     // for the coordinates; the charges, first read by the gather after the sort, arrive meanwhile.
+    const size_t nb8 = sizeof(double) * (size_t)n, in_bytes = nb8 * (3 + c.R);
+    const bool staged = in_bytes <= kStageIn;
+    // the pinned buffer's last copy has ended by now (every call waits for the device), unless one failed half-way
+    if (staged) B200_CUDA(cudaStreamSynchronize(c.stream_in));
     B200_CUDA(cudaStreamWaitEvent(c.stream_in, c.ev_stage_free, 0));
-    B200_CUDA(cudaMemcpyAsync(c.d_stage, x, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
-    B200_CUDA(cudaMemcpyAsync(c.d_stage + n, y, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
-    B200_CUDA(cudaMemcpyAsync(c.d_stage + 2 * n, z, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
-    B200_CUDA(cudaEventRecord(c.ev_in_xyz, c.stream_in));
-    B200_CUDA(cudaMemcpyAsync(c.d_stage + 3 * n, q, sizeof(double) * n * c.R, cudaMemcpyHostToDevice, c.stream_in));
-    B200_CUDA(cudaEventRecord(c.ev_in_q, c.stream_in));
+    if (staged && ensure_stage(c, in_bytes) == B200FMM_OK) {
+      char *h = (char *)c.h_stage;
+      std::memcpy(h, x, nb8);
+      std::memcpy(h + nb8, y, nb8);
+      std::memcpy(h + 2 * nb8, z, nb8);
+      std::memcpy(h + 3 * nb8, q, nb8 * c.R);
+      B200_CUDA(cudaMemcpyAsync(c.d_stage, h, in_bytes, cudaMemcpyHostToDevice, c.stream_in));
+      B200_CUDA(cudaEventRecord(c.ev_in_xyz, c.stream_in));
+      B200_CUDA(cudaEventRecord(c.ev_in_q, c.stream_in));
+    } else {
+      B200_CUDA(cudaMemcpyAsync(c.d_stage, x, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
+      B200_CUDA(cudaMemcpyAsync(c.d_stage + n, y, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
+      B200_CUDA(cudaMemcpyAsync(c.d_stage + 2 * n, z, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream_in));
+      B200_CUDA(cudaEventRecord(c.ev_in_xyz, c.stream_in));
+      B200_CUDA(cudaMemcpyAsync(c.d_stage + 3 * n, q, sizeof(double) * n * c.R, cudaMemcpyHostToDevice, c.stream_in));
+      B200_CUDA(cudaEventRecord(c.ev_in_q, c.stream_in));
+    }
     B200_CUDA(cudaStreamWaitEvent(s, c.ev_in_xyz, 0));
     dx = c.d_stage;
     dy = c.d_stage + n;

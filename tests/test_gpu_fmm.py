@@ -196,6 +196,65 @@ def test_operation_masks_match_oracle(golden, ops):
             assert S.rel_l2(r[f], o[f]) < 1e-12, f
 
 
+@pytest.mark.parametrize("n,height", [
+    # around the tile of the sort (2048), the 64 tiles up to which its scatter adds up the counts itself, one and many
+    # blocks of leaves (1024), 256 blocks of leaves, and blocks of several chunks (above 2048 * 1024 items)
+    (1, 3), (2047, 4), (2049, 4), (131072, 6), (131073, 6), (300001, 7), (700000, 8), (2300000, 7),
+])
+def test_tree_over_sizes_matches_numpy(n, height):
+    rng = np.random.default_rng(n)
+    pos = rng.random((3, n))
+    pos[:, : n // 3] = 0.5 + 0.02 * (pos[:, : n // 3] - 0.5)  # a dense part
+    f = S.FMM("cheb_dense", 3, height)
+    f.set_particles(pos[0], pos[1], pos[2], np.ones(n))
+    perm = f.permutation()
+    counts, _ = f.tree_info()
+    leaf_keys = f.cells(height - 1, expansions=False)[0]
+    start = np.zeros(int(counts[-1]) + 1, np.int64)
+    S._check(S.lib().b200fmm_get_leaf_ranges(f._h, S._ptr(start, S._lp)), "get_leaf_ranges")
+    side = 1 << (height - 1)
+    cell = np.minimum((pos / (1.0 / side)).astype(np.int64), side - 1)
+    key = np.zeros(n, np.int64)
+    for b in range(height - 1):
+        for axis, place in ((2, 0), (1, 1), (0, 2)):
+            key |= ((cell[axis] >> b) & 1) << (3 * b + place)
+    order = np.argsort(key, kind="stable")
+    assert (perm == order).all()
+    uniq, first = np.unique(key[order], return_index=True)
+    assert (leaf_keys == uniq).all() and (start[:-1] == first).all() and start[-1] == n
+    for level in range(height - 1, -1, -1):
+        assert counts[level] == uniq.size
+        if level >= 2:
+            assert (f.cells(level, expansions=False)[0] == uniq).all()
+        uniq = np.unique(uniq >> 3)
+    f.close()
+
+
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (8192, 1), (8193, 1), (131072, 1), (131073, 1), (3000, 3)])
+def test_host_arrays_equal_device_arrays(n, nrhs):
+    """Host inputs and results up to and past the sizes that go through the pinned staging buffer."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(5)
+    x, y, z = rng.random((3, n))
+    q = rng.uniform(-1, 1, nrhs * n)
+    f = S.FMM("cheb_dense", 3, 4, nrhs=nrhs)
+    got = []
+    for _ in range(2):
+        f.set_particles(x, y, z, q)
+        f.execute()
+        got.append(f.results())
+    d = [torch.from_numpy(a).cuda() for a in (x, y, z, q)]
+    out = [torch.zeros(nrhs * n, dtype=torch.float64, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    f.set_particles(*d)
+    f.execute()
+    f.results_into(*out)
+    f.synchronize()
+    f.close()
+    for k, o in zip(FIELDS, out):
+        assert (got[0][k].ravel() == o.cpu().numpy()).all() and (got[1][k] == got[0][k]).all()
+
+
 @pytest.mark.parametrize("precision,nrhs", [("fp64", 1), ("fp64", 3), ("fp64", 5), ("mixed", 1), ("mixed", 3)])
 @pytest.mark.parametrize("variant", [0, 1])
 def test_near_field_over_leaf_sizes(precision, nrhs, variant):
