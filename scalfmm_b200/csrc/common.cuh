@@ -138,7 +138,8 @@ struct Context {
   // each a work item of its own (the last entry is the item count), so that dense leaves spread over many warps
   long long *d_chunk_base = nullptr;
   int p2p_whole = kP2PWholeLeaf, p2p_item = kP2PItemTargets;  // the work-item rule d_chunk_base was built with
-  double *d_phi = nullptr, *d_fx = nullptr, *d_fy = nullptr, *d_fz = nullptr;  // [R][N] sorted results
+  double4 *d_res = nullptr;                               // [R][N] sorted results: potential, then the forces
+  int *d_iperm = nullptr;                                 // original -> sorted
   Level lv[kMaxHeight];
   bool has_particles = false;
   bool packed32 = false;      // d_pq32 holds the current particles
@@ -326,6 +327,16 @@ __device__ inline int find_key(const long long *keys, long long n, long long key
 // Timing event k on the handle's stream, except while execute() is being captured into a CUDA graph.
 inline cudaError_t record_event(Context &c, int k) {
   return c.capturing ? cudaSuccess : cudaEventRecord(c.ev[k], c.stream);
+}
+
+// One particle's results: the near field and L2P add into them, 32 bytes at a time.
+__device__ __forceinline__ void add_result(double4 *res, double p, double x, double y, double z) {
+  double4 v = *res;
+  v.x += p;
+  v.y += x;
+  v.z += y;
+  v.w += z;
+  *res = v;
 }
 
 inline unsigned grid_for(long long n, int block) {

@@ -354,8 +354,7 @@ __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
     const long long *__restrict__ leaf_start, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, const double *__restrict__ q, double cx0, double cy0, double cz0, double leaf_w,
     const double *__restrict__ L,
-    double *__restrict__ phi, double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz,
-    const long long *__restrict__ shard) {
+    double4 *__restrict__ res, const long long *__restrict__ shard) {
   constexpr int p = P, nn = P * P * P;
   __shared__ double sL[L2P_WARPS][nn];
   __shared__ double sW[L2P_WARPS][32][4 * P + 1];  // wy, dwy, wz, dwz of each lane's particle (+1: banks)
@@ -425,10 +424,7 @@ __global__ void __launch_bounds__(L2P_WARPS * 32) l2p_kernel(
       if (on) {
         const long long j = (long long)r * N + i;
         const double qq = q[j];
-        phi[j] += pv;
-        fx[j] += gx * jac * qq;
-        fy[j] += gy * jac * qq;
-        fz[j] += gz * jac * qq;
+        add_result(res + j, pv, gx * jac * qq, gy * jac * qq, gz * jac * qq);
       }
     }
   }
@@ -535,12 +531,12 @@ b200fmm_status run_l2p(Context &c, const long long *shard) {
   case PV:                                                                                                   \
     if (lagr)                                                                                                \
       l2p_kernel<PV, true><<<grid_for(L.n, L2P_WARPS), L2P_WARPS * 32, 0, c.stream>>>(                      \
-          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.L, c.d_phi,       \
-          c.d_fx, c.d_fy, c.d_fz, shard);                                          \
+          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.L, c.d_res,       \
+          shard);                                                                                            \
     else                                                                                                     \
       l2p_kernel<PV, false><<<grid_for(L.n, L2P_WARPS), L2P_WARPS * 32, 0, c.stream>>>(                     \
-          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.L, c.d_phi,       \
-          c.d_fx, c.d_fy, c.d_fz, shard);                                          \
+          c.R, c.N, L.n, L.keys, c.d_leaf_start, c.d_x, c.d_y, c.d_z, c.d_q, x0, y0, z0, lw, L.L, c.d_res,       \
+          shard);                                                                                            \
     break;
   switch (c.p) {
     B200_L2P(3) B200_L2P(4) B200_L2P(5) B200_L2P(6) B200_L2P(7) B200_L2P(8)

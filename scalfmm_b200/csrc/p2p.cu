@@ -59,8 +59,8 @@ template <int NR>
 __global__ void __launch_bounds__(P2P64_THREADS) p2p_fp64_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     const long long *__restrict__ chunk_base, int variant, const double *__restrict__ x, const double *__restrict__ y,
-    const double *__restrict__ z, const double *__restrict__ q, double *__restrict__ phi, double *__restrict__ fx,
-    double *__restrict__ fy, double *__restrict__ fz, const long long *__restrict__ shard) {
+    const double *__restrict__ z, const double *__restrict__ q, double4 *__restrict__ res,
+    const long long *__restrict__ shard) {
   __shared__ __align__(32) double4 src[P2P64_THREADS];              // x, y, z, q (of the only right-hand side)
   __shared__ double srcq[NR > 1 ? NR : 1][NR > 1 ? P2P64_THREADS : 1];
   __shared__ double red[P2P64_WARPS - 1][4][32];
@@ -164,10 +164,7 @@ __global__ void __launch_bounds__(P2P64_THREADS) p2p_fp64_kernel(
           for (int u = 0; u < P2P64_WARPS - 1; ++u) v[c] += red[u][c][lane];
         const long long j = (long long)(r0 + r) * N + t0 + tl;
         const double nq = -q[j];
-        phi[j] += v[0];
-        fx[j] += nq * v[1];
-        fy[j] += nq * v[2];
-        fz[j] += nq * v[3];
+        add_result(res + j, v[0], nq * v[1], nq * v[2], nq * v[3]);
       }
     }
   }
@@ -400,13 +397,30 @@ __device__ __forceinline__ bool p2p_item(long long item, long long nleaves, cons
 // slots in use, and 33..48 as 32 and the rest.
 __device__ __forceinline__ int p2p_chunk(long long left) { return left > 48 ? 64 : left > 16 ? 32 : left > 8 ? 16 : 8; }
 
+// Where the results go: the handle's records, or a caller's four arrays (the allocation-free entry point).
+struct OutRecords {
+  double4 *res;
+  __device__ __forceinline__ void add(long long j, double p, double x, double y, double z) const {
+    add_result(res + j, p, x, y, z);
+  }
+};
+struct OutArrays {
+  double *phi, *fx, *fy, *fz;
+  __device__ __forceinline__ void add(long long j, double p, double x, double y, double z) const {
+    phi[j] += p;
+    fx[j] += x;
+    fy[j] += y;
+    fz[j] += z;
+  }
+};
+
+template <class Out>
 __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
     const long long *__restrict__ chunk_base, int whole, int isize, const long long *__restrict__ shard,
     const float4 *__restrict__ pq,
-    const float4 *__restrict__ plo, const float4 *__restrict__ src, double *__restrict__ phi, double *__restrict__ fx, double *__restrict__ fy,
-    double *__restrict__ fz, int *__restrict__ status) {
+    const float4 *__restrict__ plo, const float4 *__restrict__ src, const Out out, int *__restrict__ status) {
   __shared__ __align__(128) float4 buf[P2P32_WARPS][P2P32_NBUF][4 * P2P32_STAGE];
   __shared__ __align__(8) unsigned long long bar[P2P32_WARPS][P2P32_NBUF];
   __shared__ long long rbase[P2P32_WARPS][27];
@@ -572,10 +586,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
           double v[4];
 #pragma unroll
           for (int c = 0; c < 4; ++c) v[c] = u == 0 ? (double)hi[c].x + (double)lo[c].x : (double)hi[c].y + (double)lo[c].y;
-          phi[j] += v[0];
-          fx[j] += nq * v[1];
-          fy[j] += nq * v[2];
-          fz[j] += nq * v[3];
+          out.add(j, v[0], nq * v[1], nq * v[2], nq * v[3]);
         }
       }
       tb += m;
@@ -689,8 +700,7 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
     const long long *__restrict__ chunk_base, int whole, int isize, const long long *__restrict__ shard,
     const float4 *__restrict__ pq, const float4 *__restrict__ plo, const float *__restrict__ qt,
     const float4 *__restrict__ src,
-    double *__restrict__ phi, double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz,
-    int *__restrict__ status) {
+    double4 *__restrict__ res, int *__restrict__ status) {
   __shared__ __align__(128) float4 buf[P2P32_WARPS][P2P32_NBUF][MR_REC * MR_STAGE];
   __shared__ __align__(8) unsigned long long bar[P2P32_WARPS][P2P32_NBUF];
   __shared__ long long rbase[P2P32_WARPS][27];
@@ -848,10 +858,8 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
         if (active && g == 0 && r < R) {
           const long long j = (long long)r * N + i;
           const double tq = -(double)qt[j];
-          phi[j] += (double)ph_hi[k] + (double)ph_lo[k];
-          fx[j] += tq * ((double)gx_hi[k] + (double)gx_lo[k]);
-          fy[j] += tq * ((double)gy_hi[k] + (double)gy_lo[k]);
-          fz[j] += tq * ((double)gz_hi[k] + (double)gz_lo[k]);
+          add_result(res + j, (double)ph_hi[k] + (double)ph_lo[k], tq * ((double)gx_hi[k] + (double)gx_lo[k]),
+                     tq * ((double)gy_hi[k] + (double)gy_lo[k]), tq * ((double)gz_hi[k] + (double)gz_lo[k]));
         }
       }
     }
@@ -887,7 +895,7 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     B200_CUDA(record_event(c, 10));
     p2p_fp32_mrhs_kernel<<<dim3(blocks, (c.R + MR_G - 1) / MR_G), P2P32_WARPS * 32, 0, c.stream>>>(
         c.R, c.N, L.n, c.d_leaf_start, c.d_leaf_nbr, variant, c.d_leaf_rank, c.d_rec_base, c.d_chunk_base, c.p2p_whole,
-        c.p2p_item, shard, hi, lo, qt, src, c.d_phi, c.d_fx, c.d_fy, c.d_fz, c.d_status);
+        c.p2p_item, shard, hi, lo, qt, src, c.d_res, c.d_status);
     B200_CUDA(record_event(c, 11));
     ++c.launches;
   } else if (c.cfg.precision == B200FMM_MIXED) {
@@ -910,7 +918,7 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     B200_CUDA(record_event(c, 10));
     p2p_fp32_kernel<<<blocks, P2P32_WARPS * 32, 0, c.stream>>>(
         c.R, c.N, L.n, c.d_leaf_start, c.d_leaf_nbr, variant, c.d_leaf_rank, c.d_rec_base, c.d_chunk_base, c.p2p_whole,
-        c.p2p_item, shard, hi, lo, src, c.d_phi, c.d_fx, c.d_fy, c.d_fz, status);
+        c.p2p_item, shard, hi, lo, src, OutRecords{c.d_res}, status);
     B200_CUDA(record_event(c, 11));
     ++c.launches;
   } else {
@@ -923,7 +931,7 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     const unsigned blocks = grid_for(L.n + c.N / P2P64_TGT, 1);
     auto kernel = c.R > 1 ? p2p_fp64_kernel<4> : p2p_fp64_kernel<1>;
     kernel<<<blocks, P2P64_THREADS, 0, c.stream>>>(c.R, c.N, L.n, c.d_leaf_start, c.d_leaf_nbr, c.d_chunk_base, variant,
-                                                   c.d_x, c.d_y, c.d_z, c.d_q, c.d_phi, c.d_fx, c.d_fy, c.d_fz, shard);
+                                                   c.d_x, c.d_y, c.d_z, c.d_q, c.d_res, shard);
     B200_CUDA(record_event(c, 11));
     ++c.launches;
   }
@@ -1030,7 +1038,7 @@ extern "C" b200fmm_status b200fmm_p2p_noalloc(long long n, const double *x, cons
                                                  center[2] - box_width / 2, stage, stage + n, stage + 2 * n);
   p2p_fp32_kernel<<<grid_for(nleaves, P2P32_WARPS), P2P32_WARPS * 32, 0, s>>>(
       1, n, nleaves, leaf_start, leaf_nbr, variant, nullptr, nullptr, nullptr, 0, 0, nullptr, stage, stage + n,
-      stage + 2 * n, phi, fx, fy, fz, status);
+      stage + 2 * n, OutArrays{phi, fx, fy, fz}, status);
   B200_CUDA(cudaGetLastError());
   B200_CUDA(cudaMemcpyAsync(st, status, sizeof(st), cudaMemcpyDeviceToHost, s));
   B200_CUDA(cudaStreamSynchronize(s));

@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs8_scatter(const unsigned long lo
 __global__ void gather_particles(long long n, int R, const int *__restrict__ perm, const double *__restrict__ x,
                                  const double *__restrict__ y, const double *__restrict__ z,
                                  const double *__restrict__ q, double *__restrict__ xs, double *__restrict__ ys,
-                                 double *__restrict__ zs, double *__restrict__ qs, long long *__restrict__ perm64) {
+                                 double *__restrict__ zs, double *__restrict__ qs, long long *__restrict__ perm64,
+                                 int *__restrict__ iperm) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long j = perm[i];
@@ -224,6 +225,7 @@ __global__ void gather_particles(long long n, int R, const int *__restrict__ per
   zs[i] = z[j];
   for (int r = 0; r < R; ++r) qs[(long long)r * n + i] = q[(long long)r * n + j];
   perm64[i] = j;
+  iperm[j] = (int)i;
 }
 
 __global__ void gather_charges(long long n, int R, const long long *__restrict__ perm, const double *__restrict__ q,
@@ -326,7 +328,7 @@ void add_state(ClearList &cl, Context &c) {
     cl.add(c.lv[l].M, bytes, false);
     cl.add(c.lv[l].L, bytes, false);
   }
-  for (double *p : {c.d_phi, c.d_fx, c.d_fy, c.d_fz}) cl.add(p, sizeof(double) * (size_t)c.N * c.R, false);
+  cl.add(c.d_res, sizeof(double4) * (size_t)c.N * c.R, false);
 }
 
 // ---- upper levels of the tree, all at once from the sorted leaf keys ---------------------------------
@@ -655,10 +657,8 @@ void free_tree(Context &c) {
   dfree(c.d_rec_base);
   dfree(c.d_chunk_base);
   dfree(c.d_pq32);
-  dfree(c.d_phi);
-  dfree(c.d_fx);
-  dfree(c.d_fy);
-  dfree(c.d_fz);
+  dfree(c.d_res);
+  dfree(c.d_iperm);
   dfree(c.d_sortk);
   dfree(c.d_sortv);
   dfree(c.d_flags);
@@ -737,10 +737,12 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
   B200_CHECK(grow(c, c.d_z, cap, (size_t)n));
   cap = c.cap_N;
   B200_CHECK(grow(c, c.d_perm, cap, (size_t)n));
-  for (double **p : {&c.d_q, &c.d_phi, &c.d_fx, &c.d_fy, &c.d_fz}) {
-    size_t cr = c.cap_N * c.R;
-    B200_CHECK(grow(c, *p, cr, (size_t)n * c.R));
-  }
+  cap = c.cap_N;
+  B200_CHECK(grow(c, c.d_iperm, cap, (size_t)n));
+  cap = c.cap_N * c.R;
+  B200_CHECK(grow(c, c.d_q, cap, (size_t)n * c.R));
+  cap = c.cap_N * c.R;
+  B200_CHECK(grow(c, c.d_res, cap, (size_t)n * c.R));
   {
     // FP32 P2P copies: target hi [R][N], target lo [N], pair-packed sources [R][N+2][4]
     size_t cp = c.cap_N * (c.R + 1) + 4 * c.R * (c.cap_N + 2);
@@ -812,7 +814,8 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
   // stable LSD radix sort of (key, original index)
   B200_CHECK(radix_sort(c, k0, k1, v0, v1, n, 3 * LL, totals, true, c.tree_launches));
   if (!on_device) B200_CUDA(cudaStreamWaitEvent(s, c.ev_in_q, 0));
-  gather_particles<<<grid_for(n, 256), 256, 0, s>>>(n, c.R, v0, dx, dy, dz, dq, c.d_x, c.d_y, c.d_z, c.d_q, c.d_perm);
+  gather_particles<<<grid_for(n, 256), 256, 0, s>>>(n, c.R, v0, dx, dy, dz, dq, c.d_x, c.d_y, c.d_z, c.d_q, c.d_perm,
+                                                 c.d_iperm);
   B200_CUDA(cudaEventRecord(c.ev_stage_free, s));  // the last reader of the staging buffer
   // the cell count of every level at once (and the leaf heads), then the build's one synchronisation
   unsigned long long *counts = (unsigned long long *)(c.d_err + 4);
