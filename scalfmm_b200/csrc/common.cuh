@@ -329,6 +329,12 @@ inline cudaError_t record_event(Context &c, int k) {
   return c.capturing ? cudaSuccess : cudaEventRecord(c.ev[k], c.stream);
 }
 
+// Whether the work queued on the handle's stream goes into a graph: the handle's own, or one that the caller captures.
+inline bool stream_captured(const Context &c) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return c.capturing || (cudaStreamIsCapturing(c.stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone);
+}
+
 // One particle's results: the near field and L2P add into them, 32 bytes at a time.
 __device__ __forceinline__ void add_result(double4 *res, double p, double x, double y, double z) {
   double4 v = *res;

@@ -82,6 +82,7 @@ struct Sym64 {
   double *d_d = nullptr;             // [rhs][pairs of a chunk of slots][p^3]
   size_t cap_psrc = 0, cap_ppos = 0, cap_d = 0;
   // per tree
+  long long room_serial = -1;        // the tree that d_plist, d_pblk and d_y have been settled for (tree_room)
   long long list_serial = -1;
   int *d_plist = nullptr;            // cells of every level grouped by parity, in Morton order
   int *d_ptab = nullptr;             // [kMaxHeight * 8] counts, list starts, then [kMaxHeight * 8 + 1] first tiles
@@ -89,9 +90,8 @@ struct Sym64 {
   size_t cap_list = 0, cap_pblk = 0;
   double *d_y = nullptr;             // [rhs][ncells][ystride]
   size_t cap_y = 0;
-  double *d_part = nullptr;          // partial sums of split tiles
+  double *d_part = nullptr;          // partial sums of split tiles: part_slots of them, allocated once
   int *d_tick = nullptr;             // arrivals per split tile
-  size_t cap_part = 0, cap_tick = 0;
 };
 
 namespace {
@@ -888,11 +888,51 @@ constexpr size_t kYBatch = (size_t)2 << 30;   // several right-hand sides share 
 template <class T>
 b200fmm_status grow64(T *&p, size_t &cap, size_t n) {
   if (p && n <= cap) return B200FMM_OK;
-  if (p) cudaFree(p);
+  if (p) B200_CUDA(cudaFree(p));
   p = nullptr;
   cap = 0;
   B200_CUDA(cudaMalloc((void **)&p, sizeof(T) * std::max<size_t>(n, 1)));
   cap = n;
+  return B200FMM_OK;
+}
+
+// CTAs that share the K ranges of split tiles: about four per resident slot (two per SM).  tiles * split stays at or
+// below this, so that partial sums for so many serve every call and never move.
+long long part_slots(const Context &c) { return 4LL * 2 * sm_count(c); }
+
+// The buffers of the current tree's M2L: settled by its first call, for all levels and for each alone, and kept until
+// the next tree, so that none that a captured evaluation holds moves.  Nothing is allocated inside a capture: there
+// the buffers of an earlier tree serve where they are large enough, else B200FMM_ERR_UNSUPPORTED.
+b200fmm_status tree_room(Context &c) {
+  Sym64 &s = *c.s64;
+  if (s.room_serial == c.tree_serial) return B200FMM_OK;
+  const size_t per = sizeof(double) * (size_t)s.ystride;
+  size_t total = 0, blocks = 0, largest = 0;  // largest: cells of the largest level within the cap
+  for (int l = 2; l < c.H; ++l) {
+    const size_t n = (size_t)c.lv[l].n;
+    total += n;
+    blocks += (n + PB_CELLS - 1) / PB_CELLS;
+    if (per * n <= kYCap) largest = std::max(largest, n);
+  }
+  if (stream_captured(c)) {
+    if (s.cap_list < total || s.cap_pblk < blocks * 8 || (!s.dense && s.cap_y < largest * s.ystride))
+      return fail(B200FMM_ERR_UNSUPPORTED, "FP64 M2L: its buffers are allocated by an evaluation that is not captured");
+  } else {
+    B200_CHECK(grow64(s.d_plist, s.cap_list, total));
+    B200_CHECK(grow64(s.d_pblk, s.cap_pblk, blocks * 8));
+    if (!s.dense) {
+      // Y of every level, of as many right-hand sides as share a launch; fewer where there is no room for that
+      b200fmm_status st = B200FMM_ERR_OOM;
+      if (per * total <= kYCap)
+        for (size_t rb = std::min<size_t>(c.R, std::max<size_t>(1, kYBatch / std::max<size_t>(1, per * total)));
+             rb > 0 && st != B200FMM_OK; rb /= 2) {
+          st = grow64(s.d_y, s.cap_y, rb * total * s.ystride);
+          if (st != B200FMM_OK) cudaGetLastError();
+        }
+      if (st != B200FMM_OK) B200_CHECK(grow64(s.d_y, s.cap_y, largest * s.ystride));
+    }
+  }
+  s.room_serial = c.tree_serial;
   return B200FMM_OK;
 }
 
@@ -915,8 +955,6 @@ b200fmm_status parity_lists(Context &c) {
     blocks += (int)((c.lv[l].n + PB_CELLS - 1) / PB_CELLS);
   }
   la.blk0[LL + 1] = blocks;
-  B200_CHECK(grow64(s.d_plist, s.cap_list, (size_t)total));
-  B200_CHECK(grow64(s.d_pblk, s.cap_pblk, (size_t)blocks * 8));
   parity_count_kernel<<<blocks, PB_THREADS, 0, c.stream>>>(la, s.d_pblk);
   parity_scan_kernel<<<1, 256, 0, c.stream>>>(la, s.d_pblk, s.d_ptab);
   parity_place_kernel<<<blocks, PB_THREADS, 0, c.stream>>>(la, s.d_pblk, s.d_ptab, s.d_plist);
@@ -970,16 +1008,13 @@ b200fmm_status gemm64_levels(Context &c, int l0, int l1) {
   a.l1 = l1;
   a.list = s.d_plist;
   a.tab = s.d_ptab;
+  // right-hand sides that share a launch: as many as Y's room holds (tree_room)
   int rb = c.R;
   const size_t ycells = (size_t)cells * s.ystride;
   if (!s.dense) {
-    // right-hand sides that share a launch; a smaller share where the memory for Y is not there
-    rb = (int)std::min<size_t>(c.R, std::max<size_t>(1, kYBatch / (sizeof(double) * ycells)));
-    while (rb > 1 && s.cap_y < rb * ycells && grow64(s.d_y, s.cap_y, rb * ycells) != B200FMM_OK) {
-      cudaGetLastError();
-      rb = rb / 2;
-    }
-    B200_CHECK(grow64(s.d_y, s.cap_y, (size_t)rb * ycells));
+    const size_t share = std::min(s.cap_y / ycells, std::max<size_t>(1, kYBatch / (sizeof(double) * ycells)));
+    if (share == 0) return fail(B200FMM_ERR_STATE, "FP64 M2L: no room for Y");
+    rb = (int)std::min<size_t>(c.R, share);
   }
   const int mb = g_mb(c.p), nblk = (c.nn + 7) / 8;
   const int mtiles = (nblk + 2 * mb - 1) / (2 * mb);
@@ -1030,24 +1065,25 @@ b200fmm_status gemm64_levels(Context &c, int l0, int l1) {
       b.ng = (c.nn + 3) / 4;
       b.ng_inv = (unsigned)(((1ull << 32) + b.ng - 1) / b.ng);
     }
-    // K ranges per tile: about four CTAs per resident slot (two per SM) where the tiles alone are fewer
-    const long long items = tiles * mtiles * nr;
-    b.split = (int)std::max<long long>(1, std::min<long long>(kMaxSplit, 4LL * 2 * sm_count(c) / items));
-    const size_t need = (size_t)items * b.split * mb * 4 * G_THREADS;
-    if (b.split > 1 && (s.cap_part < need || s.cap_tick < (size_t)items)) {
-      // nothing can be allocated while a caller captures this stream
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      B200_CUDA(cudaStreamIsCapturing(c.stream, &cs));
-      if (cs != cudaStreamCaptureStatusNone) b.split = 1;
+    // K ranges per tile where the tiles alone are fewer than part_slots
+    const long long items = tiles * mtiles * nr, slots = part_slots(c);
+    b.split = (int)std::max<long long>(1, std::min<long long>(kMaxSplit, slots / items));
+    if (b.split > 1 && !s.d_part) {
+      const size_t part = sizeof(double) * (size_t)slots * mb * 4 * G_THREADS;
+      // nothing is allocated inside a capture; unsplit tiles also where there is no room
+      if (stream_captured(c)) {
+        b.split = 1;
+      } else if ((!s.d_tick && cudaMalloc(&s.d_tick, sizeof(int) * slots) != cudaSuccess) ||
+                 cudaMalloc(&s.d_part, part) != cudaSuccess) {
+        cudaGetLastError();
+        s.d_part = nullptr;
+        b.split = 1;
+      } else {
+        B200_CUDA(cudaMemsetAsync(s.d_tick, 0, sizeof(int) * slots, c.stream));
+      }
     }
-    if (b.split > 1) {
-      const bool fresh = s.cap_tick < (size_t)items || !s.d_tick;
-      B200_CHECK(grow64(s.d_part, s.cap_part, need));
-      B200_CHECK(grow64(s.d_tick, s.cap_tick, (size_t)items));
-      if (fresh) B200_CUDA(cudaMemsetAsync(s.d_tick, 0, sizeof(int) * s.cap_tick, c.stream));
-      b.part = s.d_part;
-      b.tick = s.d_tick;
-    }
+    b.part = s.d_part;
+    b.tick = s.d_tick;
     const dim3 grid((unsigned)(tiles * mtiles * b.split), nr);
     const size_t groups = s.dense ? 0 : (size_t)s.max_groups * sizeof(unsigned short);
     const bool v16 = !s.dense || c.nn % 2 == 0;
@@ -1167,6 +1203,7 @@ b200fmm_status dense64_tree_counts(Context &c, int *host_first) {
 
 b200fmm_status dense64_tree(Context &c, const int *host_first) {
   Sym64 &s = *c.s64;
+  B200_CHECK(tree_room(c));
   B200_CHECK(parity_lists(c));
   if (!s.pairs) return B200FMM_OK;
   for (int t = 0; t < 344; ++t) s.h_first[t] = host_first[t];
@@ -1196,7 +1233,8 @@ b200fmm_status dense64_tree(Context &c, const int *host_first) {
 }
 
 // One level, or every level with level < 0.  Returns B200FMM_ERR_UNSUPPORTED before any launch when Y of the
-// largest level of the call would exceed the cap, so that the caller keeps the per-target kernel.
+// largest level of the call would exceed the cap, or when a capture finds no buffers for this tree, so that the
+// caller keeps the per-target kernel.
 b200fmm_status run_m2l_gemm64(Context &c, int level) {
   Sym64 &s = *c.s64;
   const int LL = c.H - 1;
@@ -1209,14 +1247,11 @@ b200fmm_status run_m2l_gemm64(Context &c, int level) {
   const size_t per = sizeof(double) * (size_t)s.ystride;
   if (!s.dense && per * nmax > kYCap)
     return fail(B200FMM_ERR_UNSUPPORTED, "FP64 M2L: Y of the largest level exceeds 16 GiB");
+  B200_CHECK(tree_room(c));
   B200_CHECK(parity_lists(c));
   if (s.dense && s.pairs && level < 0) return pairs_levels(c);
-  if (s.dense || l0 == l1 || s.cap_y >= (size_t)total * s.ystride) return gemm64_levels(c, l0, l1);
   // Y of every level at once, or level by level where there is no room for that
-  if (per * total <= kYCap) {
-    if (grow64(s.d_y, s.cap_y, (size_t)total * s.ystride) == B200FMM_OK) return gemm64_levels(c, l0, l1);
-    cudaGetLastError();
-  }
+  if (s.dense || l0 == l1 || s.cap_y >= (size_t)total * s.ystride) return gemm64_levels(c, l0, l1);
   for (int l = l0; l <= l1; ++l) B200_CHECK(gemm64_levels(c, l, l));
   return B200FMM_OK;
 }

@@ -897,6 +897,48 @@ def test_repeated_execute_replays_a_graph(kernel, precision):
     f.close()
 
 
+def _full_lattice(height, per_leaf, seed):
+    """per_leaf particles in every leaf."""
+    side = 1 << (height - 1)
+    cell = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij")).reshape(3, -1).repeat(per_leaf, axis=1)
+    return (cell + np.random.default_rng(seed).uniform(0.05, 0.95, cell.shape)) / side
+
+
+@pytest.mark.parametrize("kernel,height,per_leaf,nrhs", [
+    # 97 tiles x 5: K split in 2 over all levels, in 3 for the leaf level alone, whose partial sums are more
+    ("cheb_sym", 5, 3, 5),
+    # 2 GiB hold Y of all levels for 3 right-hand sides, of the leaf level for 4, which is more
+    ("cheb_sym", 6, 2, 4),
+    # dense operators: the tile form, split
+    ("lagrange", 5, 3, 2),
+])
+def test_single_level_m2l_between_replays(kernel, height, per_leaf, nrhs):
+    """A captured evaluation stays valid when single levels, which share the launches and the K ranges out differently
+    from all levels together, run between its replays."""
+    rng = np.random.default_rng(7)
+    x, y, z = _full_lattice(height, per_leaf, 8)
+    q = rng.uniform(-1, 1, (2, nrhs * x.size))
+    f = S.FMM(kernel, 5, height, nrhs=nrhs)
+    f.set_particles(x, y, z, q[0])
+    for _ in range(2):  # the second is captured
+        f.execute()
+    assert f.timings()["m2l"] == 0
+    for level in range(height - 1, 1, -1):
+        f.m2l(level)
+    f.set_charges(q[1])
+    f.execute()
+    assert f.timings()["m2l"] == 0
+    got = f.results()
+    f.close()
+    g = S.FMM(kernel, 5, height, nrhs=nrhs)
+    g.set_particles(x, y, z, q[1])
+    g.execute()
+    want = g.results()
+    g.close()
+    for k in FIELDS:
+        assert S.rel_l2(got[k], want[k]) < 1e-13, (k, S.rel_l2(got[k], want[k]))
+
+
 @pytest.mark.parametrize("kernel,precision,tol", [("cheb_sym", "fp64", 1e-12), ("cheb_sym", "mixed", 1e-10),
                                                   ("lagrange", "mixed", 1e-10)])
 def test_batch_matches_single_problems(kernel, precision, tol):
