@@ -110,7 +110,8 @@ B200FMM_API b200fmm_status b200fmm_set_charges(b200fmm_handle h, const double *q
  * expansions and results, then runs the passes selected by ops.  The second execute() with the same ops on
  * one tree (after set_charges(), say) captures the passes into a CUDA graph, and later ones replay it with
  * a single launch; set_particles() drops it.  Environment B200FMM_GRAPHS=0 keeps every call on plain
- * launches.  A stream that the caller is capturing always gets plain launches. */
+ * launches.  A stream that the caller is capturing always gets plain launches, which build
+ * the per-tree tables that they need in the caller's graph too. */
 B200FMM_API b200fmm_status b200fmm_execute(b200fmm_handle h, unsigned ops);
 
 /* Autotuner (MIXED), on the current tree; the choices are kept by the handle:

@@ -397,8 +397,8 @@ static b200fmm_status execute_body(Context &c, unsigned ops) {
   c.launches = 0;
   const int LL = c.H - 1;
   B200_CHECK(record(c, 0));
-  // skipped right after set_particles, which zeroed them; always part of a captured graph
-  if (!c.state_zero || c.capturing) B200_CHECK(clear_state(c));
+  // skipped right after set_particles, which zeroed them; always part of a graph
+  if (!c.state_zero || stream_captured(c)) B200_CHECK(clear_state(c));
   c.state_zero = false;
   // MIXED records the multipole maxima during a full upward pass for the tensor-core M2L
   c.mmax_out = nullptr;
@@ -523,7 +523,7 @@ b200fmm_status b200fmm_execute(b200fmm_handle h, unsigned ops) {
   }
   c.last_was_graph = false;
   B200_CHECK(execute_body(c, ops));
-  if (c.eager_ops != ~0u || c.eager_serial != c.tree_serial) {
+  if (cs == cudaStreamCaptureStatusNone && (c.eager_ops != ~0u || c.eager_serial != c.tree_serial)) {
     c.eager_serial = c.tree_serial;
     c.eager_ops = ops;
   }

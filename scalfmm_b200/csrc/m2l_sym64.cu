@@ -936,7 +936,7 @@ b200fmm_status tree_room(Context &c) {
   return B200FMM_OK;
 }
 
-// Parity lists of the current tree, once per tree.
+// Parity lists of the current tree, once per tree (a graph builds its own).
 b200fmm_status parity_lists(Context &c) {
   Sym64 &s = *c.s64;
   if (s.list_serial == c.tree_serial) return B200FMM_OK;
@@ -960,7 +960,7 @@ b200fmm_status parity_lists(Context &c) {
   parity_place_kernel<<<blocks, PB_THREADS, 0, c.stream>>>(la, s.d_pblk, s.d_ptab, s.d_plist);
   c.launches += 3;
   B200_CUDA(cudaGetLastError());
-  s.list_serial = c.tree_serial;
+  if (!stream_captured(c)) s.list_serial = c.tree_serial;
   return B200FMM_OK;
 }
 

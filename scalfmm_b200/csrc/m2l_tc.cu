@@ -2745,7 +2745,9 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
   // Modes of a level's Y: 1 tile-mode rows (kept clear by the tile flags), 2 compacted first product by grid
   // position, 3 by compacted row (the gathers read only rows of cells, so leftovers elsewhere are never read).
   // Leaving mode 2 for 1 or 2 clears the earlier tree's rows; leaving mode 3 for 1 or 2, or turning from 1 to 2,
-  // clears Y and the tile flags.
+  // clears Y and the tile flags.  A caller's capture (of trees without compacted levels: the counts above end one)
+  // records these clears and leaves the modes as they are, since it has not run.
+  const bool captured = stream_captured(c);
   if (t.lr) {
     CPlace chunks{};
     for (int p = 0; p <= 8; ++p) chunks.blk0[p] = p < 8 ? t.ybase[p] : t.ycht;
@@ -2762,10 +2764,11 @@ static b200fmm_status compact_setup(Context &c, DenseTC &t) {
         B200_CUDA(cudaMemsetAsync(t.Ylo[l], 0, t.Ybytes[l], c.stream));
         B200_CUDA(cudaMemsetAsync(t.ydirty + 16 * (size_t)t.titem0[l], 0, 16 * (size_t)t.tnitems[l], c.stream));
       }
-      t.ymode[l] = next;
+      if (!captured) t.ymode[l] = next;
     }
   }
-  for (int l = 2; l <= LL; ++l) t.crows[l] = 0;
+  if (!captured)
+    for (int l = 2; l <= LL; ++l) t.crows[l] = 0;
   // rows and cells of every placed level
   CBlocks B{};
   B.l0 = 2;
@@ -2944,7 +2947,7 @@ b200fmm_status tc_tree_setup(Context &c) {
     }
     ++c.launches;
     B200_CUDA(cudaGetLastError());
-    t->sat_serial = c.tree_serial;
+    if (!stream_captured(c)) t->sat_serial = c.tree_serial;
   }
   return B200FMM_OK;
 }

@@ -872,18 +872,20 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
   const int LL = c.H - 1;
   const Level &L = c.lv[LL];
   if (L.n == 0) return B200FMM_OK;
+  // a graph builds the tables that it needs itself: what is only captured has not run, and may never
+  const bool captured = stream_captured(c);
   if (c.cfg.precision == B200FMM_MIXED && c.R > 1) {
     // several right-hand sides: targets hi [N], lo [N], charges [R][N] (floats), then the record groups; the
     // buffer sized for the single-RHS layout of R vectors holds this one
     float4 *hi = c.d_pq32, *lo = c.d_pq32 + c.N;
     float *qt = (float *)(c.d_pq32 + 2 * c.N);
     float4 *src = c.d_pq32 + 2 * c.N + (c.N * c.R + 3) / 4;
-    if (!c.packed32) {
-      c.packed32 = true;
+    if (!c.packed32 || captured) {
       if (c.column_serial != c.tree_serial) {
         B200_CHECK(leaf_column_order(c));
-        c.column_serial = c.tree_serial;
+        if (!captured) c.column_serial = c.tree_serial;
       }
+      c.packed32 = !captured;
       const double W = c.cfg.box_width;
       pack_records32_mrhs<<<(unsigned)L.n, 64, 0, c.stream>>>(
           c.N, c.R, c.d_leaf_start, c.d_leaf_rank, c.d_rec_base, c.d_x, c.d_y, c.d_z, c.d_q, c.cfg.center[0] - W / 2,
@@ -900,12 +902,12 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
     ++c.launches;
   } else if (c.cfg.precision == B200FMM_MIXED) {
     float4 *hi = c.d_pq32, *lo = c.d_pq32 + c.N * c.R, *src = c.d_pq32 + c.N * (c.R + 1);
-    if (!c.packed32) {
-      c.packed32 = true;
+    if (!c.packed32 || captured) {
       if (c.column_serial != c.tree_serial) {
         B200_CHECK(leaf_column_order(c));
-        c.column_serial = c.tree_serial;
+        if (!captured) c.column_serial = c.tree_serial;
       }
+      c.packed32 = !captured;
       const double W = c.cfg.box_width;
       pack_records32<<<(unsigned)L.n, 64, 0, c.stream>>>(c.N, c.R, c.d_leaf_start, c.d_leaf_rank, c.d_rec_base, c.d_x,
                                                          c.d_y, c.d_z, c.d_q, c.cfg.center[0] - W / 2,
@@ -924,7 +926,7 @@ b200fmm_status run_p2p(Context &c, int variant, const long long *shard) {
   } else {
     if (c.column_serial != c.tree_serial) {
       B200_CHECK(leaf_items(c, P2P64_TGT, P2P64_TGT));
-      c.column_serial = c.tree_serial;
+      if (!captured) c.column_serial = c.tree_serial;
     }
     B200_CUDA(record_event(c, 10));
     // nleaves + N / 32 bounds the work items; several right-hand sides share a pair's geometry four at a time

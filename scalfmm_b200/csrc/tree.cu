@@ -965,7 +965,7 @@ b200fmm_status shard_ranges(Context &c) {
                                              c.d_shard);
   ++c.launches;
   B200_CUDA(cudaGetLastError());
-  c.shard_serial = c.tree_serial;
+  if (!stream_captured(c)) c.shard_serial = c.tree_serial;
   return B200FMM_OK;
 }
 

@@ -939,6 +939,62 @@ def test_single_level_m2l_between_replays(kernel, height, per_leaf, nrhs):
         assert S.rel_l2(got[k], want[k]) < 1e-13, (k, S.rel_l2(got[k], want[k]))
 
 
+@pytest.mark.parametrize("kernel,precision,nrhs", [("cheb_sym", "fp64", 1), ("lagrange", "fp64", 1), ("cheb_dense", "fp64", 2),
+                                                   ("cheb_sym", "mixed", 1), ("cheb_sym", "mixed", 3)])
+def test_evaluation_under_a_callers_capture(kernel, precision, nrhs):
+    """A caller captures the first evaluation of a tree: nothing counts as built before the graph has run.  Plain
+    evaluations after a capture that was thrown away, replays, and replays after new charges all give a fresh handle's
+    results."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(3)
+    order, height = 5, 4
+    trees = [_full_lattice(height, k, k) for k in (40, 9, 20)]
+    stream = torch.cuda.Stream()
+    f = S.FMM(kernel, order, height, nrhs=nrhs, precision=precision, stream=stream.cuda_stream)
+
+    def same(pos, q):
+        g = S.FMM(kernel, order, height, nrhs=nrhs, precision=precision)
+        g.set_particles(*pos, q)
+        g.execute()
+        got, want = f.results(), g.results()
+        g.close()
+        # FP64: sums in another order; MIXED: the same kernels
+        for k in FIELDS:
+            assert S.rel_l2(got[k], want[k]) < 1e-12, (k, S.rel_l2(got[k], want[k]))
+
+    for k, pos in enumerate(trees):
+        q = rng.uniform(-1, 1, (2, nrhs * pos.shape[1]))
+        f.set_particles(*pos, q[0])
+        if k == 0 and precision == "mixed":  # its first evaluation allocates: not captured
+            f.execute()
+            same(pos, q[0])
+            continue
+        thrown_away = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(thrown_away, stream=stream):
+            f.execute()
+        del thrown_away
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            f.execute()
+        if k != 1:  # plain evaluations first, else replays first
+            for _ in range(3):
+                f.execute()
+                same(pos, q[0])
+        for _ in range(2):
+            with torch.cuda.stream(stream):
+                graph.replay()
+            same(pos, q[0])
+        f.set_charges(q[1])
+        with torch.cuda.stream(stream):
+            graph.replay()
+        same(pos, q[1])
+        f.execute()
+        same(pos, q[1])
+        f.synchronize()
+        del graph
+    f.close()
+
+
 @pytest.mark.parametrize("kernel,precision,tol", [("cheb_sym", "fp64", 1e-12), ("cheb_sym", "mixed", 1e-10),
                                                   ("lagrange", "mixed", 1e-10)])
 def test_batch_matches_single_problems(kernel, precision, tol):
