@@ -251,14 +251,6 @@ __device__ __forceinline__ void two_sum2(float2 &hi, float2 &lo, float2 v) {
   lo = __fadd2_rn(lo, err);
 }
 
-__device__ __forceinline__ void two_sum(float &hi, float &lo, float v) {
-  const float s = hi + v;
-  const float bp = s - hi;
-  const float err = (hi - (s - bp)) + (v - bp);
-  hi = s;
-  lo += err;
-}
-
 constexpr int P2P32_WARPS = 2;   // work items per CTA (one warp each): few, so that a long one holds little else up
 constexpr int P2P32_STAGE = 56;  // source records (112 particles) per bulk-copy stage
 constexpr int P2P32_FLUSH = 24;  // records per lane whose sums enter the compensated sums together
@@ -605,7 +597,8 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
 //   charges of right-hand sides past R are zero.  Record order and runs are those of the single-RHS kernel.
 constexpr int MR_G = 4;
 constexpr int MR_REC = 5;  // float4 per record
-constexpr int MR_STAGE = 48;  // records per bulk-copy stage (32: 3.4 against 3.0 ms at 250k points x 16)
+constexpr int MR_STAGE = 48;  // records per bulk-copy stage
+constexpr int MR_FLUSH = 24;  // records of a stage whose sums enter the compensated sums together
 
 __global__ void pack_records32_mrhs(long long N, int R, const long long *__restrict__ leaf_start,
                                     const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
@@ -691,9 +684,12 @@ __device__ __forceinline__ void p2p_record_mrhs(const float4 *__restrict__ s, in
 }
 
 // One warp per work item and group of MR_G right-hand sides (grid.y): runs of records in bulk-copy stages, one target
-// per lane (two would need 64 accumulator registers more), lane groups for small leaves, per-stage two-sums.  With
-// the groups one after the other in a warp, 4,096 leaves of 61 gave 1.7 waves of long items: 3.7 -> 2.6 ms with the
-// groups on the grid, items of 32 targets and the longer stages (250k points x 16).  Two warps per CTA.
+// per lane (two would need 64 accumulator registers more), lane groups for small leaves, packed compensated sums after
+// every MR_FLUSH records of a stage.  With the groups one after the other in a warp, 4,096 leaves of 61 gave 1.7 waves
+// of long items: 3.7 -> 2.45 ms with the groups on the grid, items of 32 targets and stages of 48 records instead of 32
+// (250k points x 16).  One compensated sum per 48 records let the FP32 chains grow: against FP64 the potential's error
+// was 1.0-1.3 and the forces' 1.0-1.2 times that of one per 32 (seven clouds, 8 seeds).  With one per 24 they are
+// 0.81-1.0 and 0.88-1.0 times, for 2.56 ms.  Two warps per CTA.
 __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
     int R, long long N, long long nleaves, const long long *__restrict__ leaf_start, const int *__restrict__ nbr,
     int variant, const int *__restrict__ rank_of, const long long *__restrict__ rec_base,
@@ -766,10 +762,12 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
       const long long self_slot = 2 * self_rec + (i - t0);
       const float2 th_x = make_float2(me.x, me.x), th_y = make_float2(me.y, me.y), th_z = make_float2(me.z, me.z);
       const float2 tl_x = make_float2(mel.x, mel.x), tl_y = make_float2(mel.y, mel.y), tl_z = make_float2(mel.z, mel.z);
-      float ph_hi[MR_G], ph_lo[MR_G], gx_hi[MR_G], gx_lo[MR_G], gy_hi[MR_G], gy_lo[MR_G], gz_hi[MR_G], gz_lo[MR_G];
+      // compensated potential and force sums of the right-hand sides 2 v (.x) and 2 v + 1 (.y)
+      float2 hi[4][MR_G / 2], lo[4][MR_G / 2];
 #pragma unroll
-      for (int k = 0; k < MR_G; ++k)
-        ph_hi[k] = ph_lo[k] = gx_hi[k] = gx_lo[k] = gy_hi[k] = gy_lo[k] = gz_hi[k] = gz_lo[k] = 0.f;
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int v = 0; v < MR_G / 2; ++v) hi[c][v] = lo[c][v] = make_float2(0.f, 0.f);
       int ie = 0, ip = 0, ce = 0, cp = 0, issued = 0, done = 0;
       auto next_stage = [&](int &e, int &p0, int &n) -> bool {
         while (e < nr && p0 >= rcount[w][e]) {
@@ -810,25 +808,31 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
           return;
         }
         phase_bits ^= 1u << b;
-        float2 pv[MR_G], ax[MR_G], ay[MR_G], az[MR_G];
-#pragma unroll
-        for (int k = 0; k < MR_G; ++k) pv[k] = ax[k] = ay[k] = az[k] = make_float2(0.f, 0.f);
         const float4 *s = buf[w][b];
-        if (rself[w][ce]) {
-          const int self_rel = (int)(self_slot - 2 * (rbase[w][ce] + cp));
-          for (int k = g; k < cn; k += Gl)
-            p2p_record_mrhs<true>(s, k, self_rel, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv, ax, ay, az);
-        } else {
-#pragma unroll 2
-          for (int k = g; k < cn; k += Gl)
-            p2p_record_mrhs<false>(s, k, 0, th_x, th_y, th_z, tl_x, tl_y, tl_z, pv, ax, ay, az);
-        }
+        const bool own = rself[w][ce];
+        const int self_rel = (int)(self_slot - 2 * (rbase[w][ce] + cp));
+#pragma unroll 1
+        for (int k0 = 0; k0 < cn; k0 += MR_FLUSH) {
+          const int k1 = min(cn, k0 + MR_FLUSH);
+          float2 acc[4][MR_G];
 #pragma unroll
-        for (int k = 0; k < MR_G; ++k) {
-          two_sum(ph_hi[k], ph_lo[k], pv[k].x + pv[k].y);
-          two_sum(gx_hi[k], gx_lo[k], ax[k].x + ax[k].y);
-          two_sum(gy_hi[k], gy_lo[k], ay[k].x + ay[k].y);
-          two_sum(gz_hi[k], gz_lo[k], az[k].x + az[k].y);
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int k = 0; k < MR_G; ++k) acc[c][k] = make_float2(0.f, 0.f);
+          if (own) {
+            for (int k = k0 + g; k < k1; k += Gl)
+              p2p_record_mrhs<true>(s, k, self_rel, th_x, th_y, th_z, tl_x, tl_y, tl_z, acc[0], acc[1], acc[2], acc[3]);
+          } else {
+#pragma unroll 1  // by two: 40 bytes of spills, no faster
+            for (int k = k0 + g; k < k1; k += Gl)
+              p2p_record_mrhs<false>(s, k, 0, th_x, th_y, th_z, tl_x, tl_y, tl_z, acc[0], acc[1], acc[2], acc[3]);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int v = 0; v < MR_G / 2; ++v)
+              two_sum2(hi[c][v], lo[c][v], make_float2(acc[c][2 * v].x + acc[c][2 * v].y,
+                                                       acc[c][2 * v + 1].x + acc[c][2 * v + 1].y));
         }
         cp += cn;
         ++done;
@@ -836,30 +840,30 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_mrhs_kernel(
         issue();
       }
 #pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int v = 0; v < MR_G / 2; ++v)
+          for (int off = T; off < 32; off <<= 1) {
+            const float2 oh = make_float2(__shfl_xor_sync(0xffffffffu, hi[c][v].x, off),
+                                          __shfl_xor_sync(0xffffffffu, hi[c][v].y, off));
+            const float2 ol = make_float2(__shfl_xor_sync(0xffffffffu, lo[c][v].x, off),
+                                          __shfl_xor_sync(0xffffffffu, lo[c][v].y, off));
+            two_sum2(hi[c][v], lo[c][v], oh);
+            lo[c][v] = __fadd2_rn(lo[c][v], ol);
+          }
+#pragma unroll
       for (int k = 0; k < MR_G; ++k) {
-        for (int off = T; off < 32; off <<= 1) {
-          float oh = __shfl_xor_sync(0xffffffffu, ph_hi[k], off), ol = __shfl_xor_sync(0xffffffffu, ph_lo[k], off);
-          two_sum(ph_hi[k], ph_lo[k], oh);
-          ph_lo[k] += ol;
-          oh = __shfl_xor_sync(0xffffffffu, gx_hi[k], off);
-          ol = __shfl_xor_sync(0xffffffffu, gx_lo[k], off);
-          two_sum(gx_hi[k], gx_lo[k], oh);
-          gx_lo[k] += ol;
-          oh = __shfl_xor_sync(0xffffffffu, gy_hi[k], off);
-          ol = __shfl_xor_sync(0xffffffffu, gy_lo[k], off);
-          two_sum(gy_hi[k], gy_lo[k], oh);
-          gy_lo[k] += ol;
-          oh = __shfl_xor_sync(0xffffffffu, gz_hi[k], off);
-          ol = __shfl_xor_sync(0xffffffffu, gz_lo[k], off);
-          two_sum(gz_hi[k], gz_lo[k], oh);
-          gz_lo[k] += ol;
-        }
         const int r = MR_G * grp + k;
         if (active && g == 0 && r < R) {
           const long long j = (long long)r * N + i;
-          const double tq = -(double)qt[j];
-          add_result(res + j, (double)ph_hi[k] + (double)ph_lo[k], tq * ((double)gx_hi[k] + (double)gx_lo[k]),
-                     tq * ((double)gy_hi[k] + (double)gy_lo[k]), tq * ((double)gz_hi[k] + (double)gz_lo[k]));
+          const double nq = -(double)qt[j];
+          double v[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float2 h = hi[c][k / 2], l = lo[c][k / 2];
+            v[c] = k % 2 == 0 ? (double)h.x + (double)l.x : (double)h.y + (double)l.y;
+          }
+          add_result(res + j, v[0], nq * v[1], nq * v[2], nq * v[3]);
         }
       }
     }

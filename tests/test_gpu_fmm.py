@@ -290,6 +290,29 @@ def test_near_field_over_leaf_sizes(precision, nrhs, variant):
             assert S.rel_l2(r[name].reshape(nrhs, n)[k], -q[k] * ((d[a] * inv ** 3) @ q[k])) < tol
 
 
+def test_near_field_error_with_several_right_hand_sides():
+    """MIXED: the near field of several right-hand sides sums chains no longer than that of one (24 records of two
+    sources), so its error against FP64 is the same up to the order of the sums: within a quarter, over charges of one
+    sign in leaves of 61, whose potential the sums' rounding rules.  (Chains of 48: 1.7 times.)"""
+    n, height = 61 * 512, 4
+    err = {1: 0.0, 4: 0.0}
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        x, y, z = rng.random((3, n))
+        q = rng.random((4, n))
+        r = {}
+        for nrhs, precision in ((1, "fp64"), (1, "mixed"), (4, "mixed")):
+            f = S.FMM("cheb_dense", 3, height, nrhs=nrhs, precision=precision)
+            f.set_particles(x, y, z, q[:nrhs].ravel().copy())
+            f.zero_results()
+            f.p2p(0)
+            r[nrhs, precision] = f.results()["phi"].reshape(nrhs, n)[0]
+            f.close()
+        for nrhs in err:
+            err[nrhs] += S.rel_l2(r[nrhs, "mixed"], r[1, "fp64"])
+    assert err[4] < 1.25 * err[1], err
+
+
 @pytest.mark.parametrize("kernel,order,height,n,dist,nrhs", [
     # sizes around the 64-cell tiles and the row tiles of every order, K tails of p^3 mod 4, split and unsplit K
     ("cheb_sym", 3, 4, 700, "plummer", 1), ("cheb_sym", 4, 5, 1500, "ellipsoid", 3), ("cheb_sym", 5, 5, 9000, "uniform", 1),
