@@ -344,7 +344,7 @@ b200fmm_status b200fmm_set_particles(b200fmm_handle h, long long n, const double
   b200fmm_status st = build_tree(c, x, y, z, q, on_device != 0);
   if (st != B200FMM_OK) return st;
   c.state_zero = true;  // a new tree starts from zero expansions and results
-  // the FP64 M2L's per-tree tables for dense operators need a count from the device: it travels under the wait below
+  // the FP64 M2L's pair tables for dense operators need a count from the device: it travels under the wait below
   const bool dense64 = c.cfg.precision == B200FMM_FP64 && c.cfg.kernel != B200FMM_CHEB_SYM;
   int *dense_first = (int *)(c.h_pinned + 64);
   if (dense64) B200_CHECK(dense64_tree_counts(c, dense_first));
@@ -436,6 +436,8 @@ static b200fmm_status execute_body(Context &c, unsigned ops) {
   // the tensor-core M2L's per-tree tables (one host synchronisation on compacted levels) while the near field
   // runs on the second stream
   if (c.cfg.precision == B200FMM_MIXED && (ops & B200FMM_M2L)) B200_CHECK(tc_tree_setup(c));
+  if (c.cfg.precision == B200FMM_FP64 && c.cfg.kernel != B200FMM_CHEB_SYM && (ops & B200FMM_M2L))
+    B200_CHECK(dense64_pairs(c));
   if (ops & B200FMM_P2M) B200_CHECK(run_p2m(c));
   B200_CHECK(record(c, 2));
   if (ops & B200FMM_M2M)

@@ -265,9 +265,11 @@ b200fmm_status sym64_prepare(Context &c, const double *d_Ut, const double *d_Vt,
                              const std::vector<int> &trank);
 void sym64_free(Context &c);
 b200fmm_status dense64_prepare(Context &c);
-// dense operators: the tree's tables, queued (with the 344 words copied to the host) and then finished after a wait
+// dense operators, for each tree: the pair counts, queued (with the 344 words copied to the host) and taken after a
+// wait; the pair tables of a whole M2L
 b200fmm_status dense64_tree_counts(Context &c, int *host_first);
 b200fmm_status dense64_tree(Context &c, const int *host_first);
+b200fmm_status dense64_pairs(Context &c);
 b200fmm_status run_m2l_gemm64(Context &c, int level);
 // rows of the stacked V of each source parity (the ranks of the slots that parity feeds)
 bool sym64_fed_ranks(const Context &c, double *fed);

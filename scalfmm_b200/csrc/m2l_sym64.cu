@@ -74,7 +74,8 @@ struct Sym64 {
   double *d_a = nullptr;             // phase-2 operators, row k of slot t at (arow[t] + k) * lda; dense: d_dense
   int4 *d_ent = nullptr;             // [8][189]: (first operator row, first row of Y, K, 0) of entry e of child type ct
   // pairs grouped by transfer vector (dense operators), per tree
-  bool pairs = false;                // the tables of the current tree are there
+  bool pairs = false;                // the current tree takes the pair form
+  long long pair_serial = -1;        // the tree whose tables are there
   int *d_pairtab = nullptr;          // [344] first pair, [344] first tile, [343] counts / cursors of each slot
   int h_first[344] = {0};            // host copy of the first pair of each slot
   int *d_psrc = nullptr;             // [pairs] level << 27 | source cell
@@ -1177,9 +1178,8 @@ b200fmm_status pairs_levels(Context &c) {
 
 }  // namespace
 
-// The current tree's tables of the dense forms, so that the M2L itself allocates nothing: called at the end of
-// set_particles, first to queue the pair counts (and their copy to the host), then, once the host has waited for
-// them, to place the pairs.
+// What set_particles does for the dense forms: it queues the pair counts and their copy to the host, and once it has
+// waited for them, the buffers of the tile form are sized, so that a first evaluation may be captured.
 b200fmm_status dense64_tree_counts(Context &c, int *host_first) {
   Sym64 &s = *c.s64;
   s.pairs = false;
@@ -1203,10 +1203,17 @@ b200fmm_status dense64_tree_counts(Context &c, int *host_first) {
 
 b200fmm_status dense64_tree(Context &c, const int *host_first) {
   Sym64 &s = *c.s64;
-  B200_CHECK(tree_room(c));
-  B200_CHECK(parity_lists(c));
-  if (!s.pairs) return B200FMM_OK;
-  for (int t = 0; t < 344; ++t) s.h_first[t] = host_first[t];
+  if (s.pairs)
+    for (int t = 0; t < 344; ++t) s.h_first[t] = host_first[t];
+  return tree_room(c);
+}
+
+// The pair form's tables and D, by the first evaluation of a tree that wants the M2L of all its levels (before P2M,
+// beside the near field).  Inside a capture nothing is allocated: an evaluation that finds no tables takes the tile
+// form, as do near-field or single-level calls, which need none.
+b200fmm_status dense64_pairs(Context &c) {
+  Sym64 &s = *c.s64;
+  if (!s.pairs || s.pair_serial == c.tree_serial || stream_captured(c)) return B200FMM_OK;
   const PairArgs pa = pair_args(c);
   const long long cells = pa.start[c.H], np = s.h_first[343];
   long long largest = 1;
@@ -1227,8 +1234,9 @@ b200fmm_status dense64_tree(Context &c, const int *host_first) {
   }
   pair_kernel<true><<<grid_for(cells, PAIR_CELLS), PAIR_THREADS, 0, c.stream>>>(pa, c.d_itab, s.d_pairtab + 688,
                                                                                s.d_psrc, s.d_ppos);
-  ++c.tree_launches;
+  ++c.launches;
   B200_CUDA(cudaGetLastError());
+  s.pair_serial = c.tree_serial;
   return B200FMM_OK;
 }
 
@@ -1247,9 +1255,12 @@ b200fmm_status run_m2l_gemm64(Context &c, int level) {
   const size_t per = sizeof(double) * (size_t)s.ystride;
   if (!s.dense && per * nmax > kYCap)
     return fail(B200FMM_ERR_UNSUPPORTED, "FP64 M2L: Y of the largest level exceeds 16 GiB");
+  if (s.dense && level < 0) {
+    B200_CHECK(dense64_pairs(c));
+    if (s.pairs && s.pair_serial == c.tree_serial) return pairs_levels(c);
+  }
   B200_CHECK(tree_room(c));
   B200_CHECK(parity_lists(c));
-  if (s.dense && s.pairs && level < 0) return pairs_levels(c);
   // Y of every level at once, or level by level where there is no room for that
   if (s.dense || l0 == l1 || s.cap_y >= (size_t)total * s.ystride) return gemm64_levels(c, l0, l1);
   for (int l = l0; l <= l1; ++l) B200_CHECK(gemm64_levels(c, l, l));

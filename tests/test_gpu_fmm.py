@@ -1018,6 +1018,30 @@ def test_evaluation_under_a_callers_capture(kernel, precision, nrhs):
     f.close()
 
 
+def test_pair_tables_are_for_whole_evaluations():
+    """FP64 dense operators: the pairs' products (700 MB here) are allocated by the first M2L of all levels, not by
+    set_particles, the near field or single levels."""
+    torch = pytest.importorskip("torch")
+    n, height = 30000, 5
+    x, y, z = np.random.default_rng(9).random((3, n))
+    torch.cuda.synchronize()
+    f = S.FMM("lagrange", 5, height)
+    before = torch.cuda.mem_get_info()[0]
+    f.set_particles(x, y, z, np.ones(n))
+    f.p2p(0)
+    f.p2m()
+    for level in range(height - 2, 1, -1):
+        f.m2m(level)
+    for level in range(2, height):
+        f.m2l(level)
+    f.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 300 << 20
+    f.execute()
+    f.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] > 500 << 20
+    f.close()
+
+
 @pytest.mark.parametrize("kernel,precision,tol", [("cheb_sym", "fp64", 1e-12), ("cheb_sym", "mixed", 1e-10),
                                                   ("lagrange", "mixed", 1e-10)])
 def test_batch_matches_single_problems(kernel, precision, tol):
