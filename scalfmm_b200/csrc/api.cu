@@ -48,6 +48,18 @@ b200fmm_status ensure_stage(Context &c, size_t bytes) {
   return B200FMM_OK;
 }
 
+// Whether count arrays (nulls aside) may go through the staging buffer: not unless all are plain host memory (any other
+// pointer is left to the copy's own checks), and not page-locked ones whose bytes are above locked_limit.
+bool may_stage(const void *const *p, int count, size_t bytes, size_t locked_limit) {
+  for (int k = 0; k < count; ++k) {
+    cudaPointerAttributes a{};
+    if (!p[k]) continue;
+    if (cudaPointerGetAttributes(&a, p[k]) != cudaSuccess) cudaGetLastError();
+    if (a.type == cudaMemoryTypeHost ? bytes > locked_limit : a.type != cudaMemoryTypeUnregistered) return false;
+  }
+  return true;
+}
+
 // The status words' copy is queued behind the work that it reports; read_status() looks at it after a wait.
 static int *status_words(Context &c) { return (int *)((char *)c.h_pinned + kPinnedCounts); }
 static b200fmm_status queue_status(Context &c) {
@@ -680,7 +692,8 @@ b200fmm_status b200fmm_get_results(b200fmm_handle h, double *phi, double *fx, do
                                                               o + 2 * n * c.R, o + 3 * n * c.R);
   B200_CUDA(cudaGetLastError());
   double *dst[4] = {phi, fx, fy, fz};
-  const bool staged = 4 * bytes <= kStageOut && ensure_stage(c, 4 * bytes) == B200FMM_OK;
+  const bool staged = 4 * bytes <= kStageOut && may_stage((void **)dst, 4, 4 * bytes, 3 * kStageLocked) &&
+                      ensure_stage(c, 4 * bytes) == B200FMM_OK;
   if (staged)
     B200_CUDA(cudaMemcpyAsync(c.h_stage, o, 4 * bytes, cudaMemcpyDeviceToHost, c.stream));
   else

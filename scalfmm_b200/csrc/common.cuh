@@ -202,9 +202,12 @@ b200fmm_status check_status(Context &c);
 // Host arrays up to these sizes (all of a call's arrays together) go through the handle's pinned staging buffer.  A
 // copy from or to pageable memory costs the host 10-30 us whatever its size and waits for the device; one copy of
 // everything and a memcpy cost less up to here: a whole evaluation of 2,003 points 396 -> 349 us, of 20,000 points
-// (FP64, order 7; only its results are staged) 1,868 -> 1,775 us.
-constexpr size_t kStageIn = 256 << 10, kStageOut = 4 << 20;
+// (FP64, order 7; only its results are staged) 1,868 -> 1,775 us.  Page-locked arrays gain only the copies' latencies,
+// 2-3 us each, up to kStageLocked bytes per copy saved (four results of 8,000 points 36 us staged, 40 straight; of
+// 60,000 points 170 and 69).
+constexpr size_t kStageIn = 256 << 10, kStageOut = 4 << 20, kStageLocked = 96 << 10;
 b200fmm_status ensure_stage(Context &c, size_t bytes);
+bool may_stage(const void *const *p, int count, size_t bytes, size_t locked_limit);
 constexpr size_t kPinnedCounts = sizeof(long long) * 64 + sizeof(int) * 344;
 
 // ---- module entry points -------------------------------------------------------------------------

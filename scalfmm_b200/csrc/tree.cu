@@ -773,7 +773,8 @@ b200fmm_status build_tree(Context &c, const double *x, const double *y, const do
     // its last main-stream reader (the previous build's gather, or set_charges' gather) has run.  The keys wait
     // for the coordinates; the charges, first read by the gather after the sort, arrive meanwhile.
     const size_t nb8 = sizeof(double) * (size_t)n, in_bytes = nb8 * (3 + c.R);
-    const bool staged = in_bytes <= kStageIn;
+    const void *in[4] = {x, y, z, q};
+    const bool staged = in_bytes <= kStageIn && may_stage(in, 4, in_bytes, 3 * kStageLocked);
     // the pinned buffer's last copy has ended by now (every call waits for the device), unless one failed half-way
     if (staged) B200_CUDA(cudaStreamSynchronize(c.stream_in));
     B200_CUDA(cudaStreamWaitEvent(c.stream_in, c.ev_stage_free, 0));

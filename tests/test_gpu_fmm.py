@@ -255,6 +255,32 @@ def test_host_arrays_equal_device_arrays(n, nrhs):
         assert (got[0][k].ravel() == o.cpu().numpy()).all() and (got[1][k] == got[0][k]).all()
 
 
+@pytest.mark.parametrize("n", [2000, 9000, 40000])  # inputs and results, results alone, neither within the staging limits
+@pytest.mark.parametrize("pinned", [(), (0,), (3,), (0, 1, 2, 3)])
+def test_page_locked_arrays(n, pinned):
+    """Page-locked arrays, alone or among pageable ones, below and above the sizes that are staged."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(4)
+    data = [*rng.random((3, n)), rng.uniform(-1, 1, n)]
+    a = [torch.from_numpy(v).pin_memory() if k in pinned else torch.from_numpy(v) for k, v in enumerate(data)]
+    out = [torch.zeros(n, dtype=torch.float64, pin_memory=k in pinned) for k in range(4)]
+    f = S.FMM("cheb_dense", 3, 4)
+    for _ in range(2):
+        f.set_particles(*a)
+        f.execute()
+        f.results_into(*out)
+    g = S.FMM("cheb_dense", 3, 4)
+    d = [v.cuda() for v in a]
+    torch.cuda.synchronize()
+    g.set_particles(*d)
+    g.execute()
+    want = g.results()
+    f.close()
+    g.close()
+    for k, o in zip(FIELDS, out):
+        assert (o.numpy() == want[k]).all()
+
+
 @pytest.mark.parametrize("precision,nrhs", [("fp64", 1), ("fp64", 3), ("fp64", 5), ("mixed", 1), ("mixed", 3)])
 @pytest.mark.parametrize("variant", [0, 1])
 def test_near_field_over_leaf_sizes(precision, nrhs, variant):
