@@ -686,24 +686,30 @@ b200fmm_status b200fmm_get_results(b200fmm_handle h, double *phi, double *fx, do
     B200_CUDA(cudaGetLastError());
     return B200FMM_OK;
   }
-  B200_CHECK(ensure_scratch(c, 4 * bytes + 4096));
-  double *o = (double *)((char *)c.d_scratch + 4096);
-  results_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_iperm, c.d_res, o, o + n * c.R,
-                                                              o + 2 * n * c.R, o + 3 * n * c.R);
+  // only the wanted arrays, one after the other
+  double *dst[4] = {phi, fx, fy, fz}, *o[4] = {nullptr, nullptr, nullptr, nullptr};
+  int copies = 0;
+  for (int k = 0; k < 4; ++k) copies += dst[k] ? 1 : 0;
+  const size_t total = copies * bytes;
+  B200_CHECK(ensure_scratch(c, total + 4096));
+  char *first = (char *)c.d_scratch + 4096;
+  for (int k = 0, m = 0; k < 4; ++k)
+    if (dst[k]) o[k] = (double *)(first + bytes * m++);
+  results_to_original<<<grid_for(n, 256), 256, 0, c.stream>>>(n, c.R, c.d_iperm, c.d_res, o[0], o[1], o[2], o[3]);
   B200_CUDA(cudaGetLastError());
-  double *dst[4] = {phi, fx, fy, fz};
-  const bool staged = 4 * bytes <= kStageOut && may_stage((void **)dst, 4, 4 * bytes, 3 * kStageLocked) &&
-                      ensure_stage(c, 4 * bytes) == B200FMM_OK;
+  const bool staged = copies > 0 && total <= kStageOut &&
+                      may_stage((void **)dst, 4, total, (copies - 1) * kStageLocked) &&
+                      ensure_stage(c, total) == B200FMM_OK;
   if (staged)
-    B200_CUDA(cudaMemcpyAsync(c.h_stage, o, 4 * bytes, cudaMemcpyDeviceToHost, c.stream));
+    B200_CUDA(cudaMemcpyAsync(c.h_stage, first, total, cudaMemcpyDeviceToHost, c.stream));
   else
     for (int k = 0; k < 4; ++k)
-      if (dst[k]) B200_CUDA(cudaMemcpyAsync(dst[k], o + k * n * c.R, bytes, cudaMemcpyDeviceToHost, c.stream));
+      if (dst[k]) B200_CUDA(cudaMemcpyAsync(dst[k], o[k], bytes, cudaMemcpyDeviceToHost, c.stream));
   B200_CHECK(queue_status(c));
   B200_CUDA(cudaStreamSynchronize(c.stream));
   if (staged)
     for (int k = 0; k < 4; ++k)
-      if (dst[k]) std::memcpy(dst[k], (char *)c.h_stage + k * bytes, bytes);
+      if (dst[k]) std::memcpy(dst[k], (char *)c.h_stage + ((char *)o[k] - first), bytes);
   return read_status(c);
 }
 

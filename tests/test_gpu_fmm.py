@@ -281,6 +281,30 @@ def test_page_locked_arrays(n, pinned):
         assert (o.numpy() == want[k]).all()
 
 
+@pytest.mark.parametrize("n", [3001, 50001])  # all four results, and one alone, below and above the staging limit
+@pytest.mark.parametrize("where", ["pageable", "pinned", "device"])
+@pytest.mark.parametrize("wanted", [(0,), (1, 3), (0, 1, 2, 3), ()])
+def test_some_results_only(n, where, wanted):
+    torch = pytest.importorskip("torch")
+    nrhs = 3
+    rng = np.random.default_rng(6)
+    x, y, z = rng.random((3, n))
+    f = S.FMM("cheb_dense", 3, 4, nrhs=nrhs)
+    f.set_particles(x, y, z, rng.uniform(-1, 1, nrhs * n))
+    f.execute()
+    want = f.results()
+    out = [torch.zeros(nrhs * n, dtype=torch.float64, device="cuda" if where == "device" else "cpu",
+                       pin_memory=where == "pinned") for _ in range(4)]
+    torch.cuda.synchronize()
+    args = [out[k].data_ptr() if k in wanted else None for k in range(4)]
+    S._check(S.lib().b200fmm_get_results(f._h, *args, 1 if where == "device" else 0), "get_results")
+    f.synchronize()
+    f.close()
+    for k, name in enumerate(FIELDS):
+        got = out[k].cpu().numpy()
+        assert (got == (want[name].ravel() if k in wanted else 0.0)).all(), name
+
+
 @pytest.mark.parametrize("precision,nrhs", [("fp64", 1), ("fp64", 3), ("fp64", 5), ("mixed", 1), ("mixed", 3)])
 @pytest.mark.parametrize("variant", [0, 1])
 def test_near_field_over_leaf_sizes(precision, nrhs, variant):
