@@ -37,7 +37,8 @@ __device__ __forceinline__ void p2p64_pair(const double4 &s, bool self, const do
   const double inv2 = inv * inv;
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
-    const double p = inv * (NR == 1 ? s.w : sq[r * sq_stride]);
+    double p = inv * (NR == 1 ? s.w : sq[r * sq_stride]);
+    if (SELF && self) p = 0.0;  // the target is left out, whatever its charge (0 times an infinite one is no number)
     const double f = p * inv2;
     pv[r] += p;
     gx[r] += dx * f;

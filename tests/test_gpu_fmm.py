@@ -363,6 +363,28 @@ def test_near_field_error_with_several_right_hand_sides():
     assert err[4] < 1.25 * err[1], err
 
 
+@pytest.mark.parametrize("nrhs", [1, 3])
+@pytest.mark.parametrize("charge", [np.inf, -np.inf, np.nan])
+def test_fp64_near_field_leaves_out_the_target_itself(nrhs, charge):
+    """A particle whose charge is not finite has the finite potential of the others at its own place."""
+    rng = np.random.default_rng(12)
+    n = 60
+    pos = 0.2 * rng.random((3, n))  # one leaf of height 3
+    q = rng.uniform(-1, 1, (nrhs, n))
+    q[0, 7] = charge
+    f = S.FMM("cheb_dense", 3, 3, nrhs=nrhs)
+    f.set_particles(*pos, q.ravel())
+    f.zero_results()
+    f.p2p(0)
+    phi = f.results()["phi"].reshape(nrhs, n)
+    f.close()
+    d = pos[:, 7, None] - np.delete(pos, 7, axis=1)
+    terms = np.delete(q, 7, axis=1) / np.sqrt((d * d).sum(axis=0))
+    # a few roundings of 1.1e-16 per term, and 59 terms
+    assert (np.abs(phi[:, 7] - terms.sum(axis=1)) < 1e-14 * np.abs(terms).sum(axis=1)).all()
+    assert not np.isfinite(np.delete(phi[0], 7)).any() and np.isfinite(phi[1:]).all()
+
+
 @pytest.mark.parametrize("kernel,order,height,n,dist,nrhs", [
     # sizes around the 64-cell tiles and the row tiles of every order, K tails of p^3 mod 4, split and unsplit K
     ("cheb_sym", 3, 4, 700, "plummer", 1), ("cheb_sym", 4, 5, 1500, "ellipsoid", 3), ("cheb_sym", 5, 5, 9000, "uniform", 1),
