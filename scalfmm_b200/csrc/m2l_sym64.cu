@@ -1087,16 +1087,18 @@ b200fmm_status gemm64_levels(Context &c, int l0, int l1) {
     b.tick = s.d_tick;
     const dim3 grid((unsigned)(tiles * mtiles * b.split), nr);
     const size_t groups = s.dense ? 0 : (size_t)s.max_groups * sizeof(unsigned short);
-    const bool v16 = !s.dense || c.nn % 2 == 0;
-#define B200_G64(MBV)                                                                                   \
-  case MBV:                                                                                             \
-    if (v16)                                                                                            \
-      B200_CHECK((launch_gemm64<MBV, G_TILES, true>(b, grid, G_STAGES * gemm64_stage_bytes<MBV>() + groups, c.stream)));   \
-    else                                                                                                \
-      B200_CHECK((launch_gemm64<MBV, G_TILES, false>(b, grid, G_STAGES * gemm64_stage_bytes<MBV>() + groups, c.stream)));  \
-    break;
-    switch (mb) {
-      B200_G64(2) B200_G64(4) B200_G64(7) B200_G64(8) B200_G64(11)
+#define B200_G64(P)                                                                \
+  case P: {                                                                        \
+    constexpr int MB = g_mb(P);                                                    \
+    const size_t sh = G_STAGES * gemm64_stage_bytes<MB>() + groups;                \
+    if (s.dense)                                                                   \
+      B200_CHECK((launch_gemm64<MB, G_TILES, P % 2 == 0>(b, grid, sh, c.stream))); \
+    else                                                                           \
+      B200_CHECK((launch_gemm64<MB, G_TILES, true>(b, grid, sh, c.stream)));       \
+    break;                                                                         \
+  }
+    switch (c.p) {
+      B200_G64(3) B200_G64(4) B200_G64(5) B200_G64(6) B200_G64(7) B200_G64(8)
       default: return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
     }
 #undef B200_G64
@@ -1154,15 +1156,16 @@ b200fmm_status pairs_levels(Context &c) {
         }
         const long long tiles = (np + G_BN - 1) / G_BN + (s1 - s0);  // bounds the tiles of these slots
         const dim3 grid((unsigned)(tiles * a.mtiles), nr);
-#define B200_G64(MBV)                                                                                              \
-  case MBV:                                                                                                        \
-    if (c.nn % 2 == 0)                                                                                             \
-      B200_CHECK((launch_gemm64<MBV, G_PAIRS, true>(a, grid, G_STAGES * gemm64_stage_bytes<MBV>(), c.stream)));    \
-    else                                                                                                           \
-      B200_CHECK((launch_gemm64<MBV, G_PAIRS, false>(a, grid, G_STAGES * gemm64_stage_bytes<MBV>(), c.stream)));   \
-    break;
-        switch (mb) {
-          B200_G64(2) B200_G64(4) B200_G64(7) B200_G64(8) B200_G64(11)
+#define B200_G64(P)                                                                       \
+  case P: {                                                                               \
+    static_assert(P >= kPairOrder, "the pair form is built for the orders that take it"); \
+    constexpr int MB = g_mb(P);                                                           \
+    const size_t sh = G_STAGES * gemm64_stage_bytes<MB>();                                \
+    B200_CHECK((launch_gemm64<MB, G_PAIRS, P % 2 == 0>(a, grid, sh, c.stream)));          \
+    break;                                                                                \
+  }
+        switch (c.p) {
+          B200_G64(5) B200_G64(6) B200_G64(7) B200_G64(8)
           default: return fail(B200FMM_ERR_UNSUPPORTED, "order not built");
         }
 #undef B200_G64
