@@ -134,10 +134,10 @@ struct Context {
   float4 *d_pq32 = nullptr;                               // FP32 near-field copies (MIXED), see p2p.cu
   int *d_leaf_rank = nullptr;      // [nleaves] position of each leaf in the column-major record order (MIXED P2P)
   long long *d_rec_base = nullptr; // [nleaves+1] first source record of each leaf, in that order
-  // [nleaves+1] first work item of each leaf in the FP32 near field (p2p_leaf_items per leaf,
-  // each a work item of its own (the last entry is the item count), so that dense leaves spread over many warps
+  // [nleaves+1] first work item of each leaf in the near field, the last entry the item count (p2p_leaf_items per leaf,
+  // so that dense leaves spread over many warps).  MIXED: by the rule p2p_whole, p2p_item; FP64: 32 targets each.
   long long *d_chunk_base = nullptr;
-  int p2p_whole = kP2PWholeLeaf, p2p_item = kP2PItemTargets;  // the work-item rule d_chunk_base was built with
+  int p2p_whole = kP2PWholeLeaf, p2p_item = kP2PItemTargets;
   double4 *d_res = nullptr;                               // [R][N] sorted results: potential, then the forces
   int *d_iperm = nullptr;                                 // original -> sorted
   Level lv[kMaxHeight];

@@ -98,10 +98,10 @@ __device__ __forceinline__ void record_max(unsigned long long *slots, double mx)
 // particles (one each) into shared memory; then thread t < p^2 owns the node line (ny, nz) = (t % p, t / p)
 // and keeps its p sums over nx in registers: per particle one product q Sy Sz and p FMAs with the
 // broadcast Sx row, instead of three shared-memory reads per node and particle.  Several right-hand sides are taken
-// two at a time, with the weights of a leaf of one chunk evaluated once (250k points x 16, order 7: 0.48 -> 0.29
-// ms: the shared-memory reads of the weights bound it).  (Measured slower, 1M uniform, order 7, height 6: 128 threads, the weights along
-// rows of particles, two particles per load and two node lines per lane, 0.250 against 0.148 ms: 96 registers with
-// spills and three more barriers per leaf cost more than the halved shared-memory reads give.)
+// two at a time, with the weights of a leaf of one chunk evaluated once (250k points x 16, order 7: 0.48 -> 0.29 ms:
+// the shared-memory reads of the weights bound it).  (Measured slower, 1M uniform, order 7, height 6: 128 threads, the
+// weights along rows of particles, two particles per load and two node lines per lane, 0.250 against 0.148 ms: 96
+// registers with spills and three more barriers per leaf cost more than the halved shared-memory reads give.)
 constexpr int P2M_THREADS = 64;
 constexpr int L2P_WARPS = 1;  // L2P: leaves per CTA, one warp each (static shared memory <= 48 KB at order 8)
 
@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(P2M_THREADS, 8) p2m_kernel(
     const long long *__restrict__ leaf_start, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, const double *__restrict__ q, double cx0, double cy0, double cz0, double leaf_w,
     double *__restrict__ M, unsigned long long *__restrict__ mmax) {
-  constexpr int p = P, nn = P * P * P, PX = P <= 6 ? (P + 1) & ~1 : 10;  // Sx rows: 16-byte steps, spread over the banks
+  constexpr int p = P, nn = P * P * P;
+  constexpr int PX = P <= 6 ? (P + 1) & ~1 : 10;  // Sx rows: 16-byte steps, spread over the banks
   __shared__ __align__(16) double Wx[P2M_THREADS][PX];
   __shared__ double Wy[P2M_THREADS][P], Wz[P2M_THREADS][P], Q[NR][P2M_THREADS];
   const int t = threadIdx.x;
@@ -439,11 +440,11 @@ b200fmm_status upload_basis_constants(const Context &c, const double *roots, con
   B200_CUDA(cudaMemcpyToSymbol(c_roots, roots, sizeof(double) * p,
                                sizeof(double) * ((size_t)(lag * (kMaxOrder - 2) + p - 3) * kMaxOrder)));
   // S [8 children][3 axes][p][p]: children 0 and 4 differ in the bit of axis 0
+  const size_t table = sizeof(double) * kMaxOrder * kMaxOrder;
   for (int bit = 0; bit < 2; ++bit)
     B200_CUDA(cudaMemcpyToSymbol(c_S, S + (size_t)bit * 4 * 3 * p * p, sizeof(double) * p * p,
-                                 sizeof(double) * ((size_t)((lag * (kMaxOrder - 2) + p - 3) * 2 + bit) * kMaxOrder * kMaxOrder)));
-  if (!lag)
-    B200_CUDA(cudaMemcpyToSymbol(c_Tr, Tr, sizeof(double) * p * p, sizeof(double) * (size_t)(p - 3) * kMaxOrder * kMaxOrder));
+                                 table * ((lag * (kMaxOrder - 2) + p - 3) * 2 + bit)));
+  if (!lag) B200_CUDA(cudaMemcpyToSymbol(c_Tr, Tr, sizeof(double) * p * p, table * (p - 3)));
   return B200FMM_OK;
 }
 

@@ -4,7 +4,7 @@
 //    reference permutes every source multipole into its symmetry class frame (pvectors, pindices), applies the
 //    16 compressed operators as Y = V^T M' then scale * U Y per class, and adds the result back through the
 //    same permutation.  Here the permutation is folded into per-slot factors U_t, V_t once (precompute.cu),
-//    and one CTA applies them for 32 targets of one child type -- which share their 189 slots -- keeping the
+//    and one CTA applies them for 16 targets of one child type -- which share their 189 slots -- keeping the
 //    local sums in registers.  Kept for trees whose Y would exceed the cap of the GEMM form (m2l_sym64.cu).
 //  * CHEB_DENSE / LAGRANGE: the GEMM form.
 //  scale = 2 / cell width (FInterpMatrixKernelR::getScaleFactor, FInterpMatrixKernel.hpp:124-133).

@@ -541,9 +541,8 @@ __global__ void __launch_bounds__(G_THREADS, 2) gemm64_kernel(const __grid_const
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
       const int c = cells[bc + u * (G_BN / NU)];
-      bp[u] = c < 0 ? nullptr
-                    : (MODE == G_PAIRS ? a.X[c >> 27] + (long long)blockIdx.y * a.xrhs + (long long)(c & 0x7ffffff) * a.xstride
-                                       : X + (long long)c * a.xstride) + bk;
+      const double *base = MODE == G_PAIRS && c >= 0 ? a.X[c >> 27] + (long long)blockIdx.y * a.xrhs : X;
+      bp[u] = c < 0 ? nullptr : base + (long long)(MODE == G_PAIRS ? c & 0x7ffffff : c) * a.xstride + bk;
     }
   }
   auto sources = [&](int st) {

@@ -11,8 +11,8 @@
 //    instructions (add/mul/fma.f32x2): positions relative to the box corner as a float pair (hi, lo), so that per pair
 //    dx = (t_hi - s_hi) + (t_lo - s_lo) with the first difference exact for nearby particles (Sterbenz),
 //    which keeps the close pairs -- the ones that dominate the forces -- accurate to a few ulp.  One warp per
-//    leaf or piece of a larger one; the neighbour leaves are walked as contiguous runs of records (one per neighbour column)
-//    copied into shared memory by the bulk-copy engine (cp.async.bulk + mbarrier, 3-deep ring); rsqrt on the
+//    leaf or piece of a larger one; the neighbour leaves are walked as contiguous runs of records (one per neighbour
+//    column) copied into shared memory by the bulk-copy engine (cp.async.bulk + mbarrier, 3-deep ring); rsqrt on the
 //    SFU; per-target compensated (two-sum) accumulation of partial sums; the result is added
 //    in FP64 to the far field.
 #include "common.cuh"
@@ -242,7 +242,7 @@ __global__ void pack_records32(long long N, int R, const long long *__restrict__
   }
 }
 
-// The same for two values at once, packed.
+// Compensated (two-sum) accumulation of two values at once, packed.
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ void two_sum2(float2 &hi, float2 &lo, float2 v) {
   const float2 s = __fadd2_rn(hi, v);
@@ -316,9 +316,12 @@ __device__ __forceinline__ void p2p_record(const float4 *__restrict__ s, int k, 
   const float4 A = s[4 * k], B = s[4 * k + 1], C = s[4 * k + 2], D = s[4 * k + 3];
 #pragma unroll
   for (int u = 0; u < P2P32_TGT; ++u) {
-    const float2 dx = __fadd2_rn(__fadd2_rn(t[u].hx, make_float2(A.x, A.y)), __fadd2_rn(t[u].lx, make_float2(C.x, C.y)));
-    const float2 dy = __fadd2_rn(__fadd2_rn(t[u].hy, make_float2(A.z, A.w)), __fadd2_rn(t[u].ly, make_float2(C.z, C.w)));
-    const float2 dz = __fadd2_rn(__fadd2_rn(t[u].hz, make_float2(B.x, B.y)), __fadd2_rn(t[u].lz, make_float2(D.x, D.y)));
+    const float2 dx =
+        __fadd2_rn(__fadd2_rn(t[u].hx, make_float2(A.x, A.y)), __fadd2_rn(t[u].lx, make_float2(C.x, C.y)));
+    const float2 dy =
+        __fadd2_rn(__fadd2_rn(t[u].hy, make_float2(A.z, A.w)), __fadd2_rn(t[u].ly, make_float2(C.z, C.w)));
+    const float2 dz =
+        __fadd2_rn(__fadd2_rn(t[u].hz, make_float2(B.x, B.y)), __fadd2_rn(t[u].lz, make_float2(D.x, D.y)));
     float2 r2 = __fmul2_rn(dx, dx);
     r2 = __ffma2_rn(dy, dy, r2);
     r2 = __ffma2_rn(dz, dz, r2);
@@ -344,14 +347,15 @@ __device__ __forceinline__ void p2p_record(const float4 *__restrict__ s, int k, 
 // stages of 56 records (the three z-neighbours of a leaf of 30 are one stage), packed compensated sums of both targets
 // after every 24 records of a lane (chains no longer than before: the error is 0.9-1.0 of the earlier kernel's) and
 // 128 registers: 1M uniform 0.885 -> 0.81 ms, 2M on a surface 6.13 -> 5.68 ms, 200k in leaves of 49 0.347 -> 0.285
-// ms.  (Five CTAs of four warps at 100 registers and stages of 44: 0.95, 5.98 and 0.31 ms.)  Sums after every 16 records cost 4 % more, after every 64 give 2 % but a larger error.
+// ms.  (Five CTAs of four warps at 100 registers and stages of 44: 0.95, 5.98 and 0.31 ms.)  Sums after every 16
+// records cost 4 % more, after every 64 give 2 % but a larger error.
 // The targets are taken 64, 32, 16 or 8 at a time (p2p_chunk); 32 (16, 8) targets occupy 16 (8, 4) lanes and are
 // replicated over 2 (4, 8) lane groups, each group walking every 2nd (4th, 8th) source record, and the groups' sums
 // are combined by shuffles at the end, so that small and ragged leaves keep the lanes busy.
 // The sources are walked as runs of contiguous records (one per neighbour column and z-adjacent group),
 // each split into stages of <= P2P32_STAGE records copied by one bulk copy into a ring of P2P32_NBUF buffers,
-// issued P2P32_NBUF - 1 stages ahead of the math.  Per stage the partial sums enter the target's (hi, lo)
-// accumulators by a two-sum.
+// issued P2P32_NBUF - 1 stages ahead of the math.  After every P2P32_FLUSH records of a lane, and at the end of a
+// stage, the partial sums enter the targets' (hi, lo) accumulators by a two-sum.
 // With chunk_base, warp (CTA x, warp w) takes the work item blockIdx.x * P2P32_WARPS + w: a leaf of at most
 // `whole` targets, or `isize` targets of a larger one (a dense leaf spreads over many warps; items past the count
 // leave at once).  Without it (the allocation-free entry point) a warp takes a whole leaf.
@@ -565,8 +569,10 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
 #pragma unroll
       for (int c = 0; c < 4; ++c)
         for (int off = T; off < 32; off <<= 1) {
-          const float2 oh = make_float2(__shfl_xor_sync(0xffffffffu, hi[c].x, off), __shfl_xor_sync(0xffffffffu, hi[c].y, off));
-          const float2 ol = make_float2(__shfl_xor_sync(0xffffffffu, lo[c].x, off), __shfl_xor_sync(0xffffffffu, lo[c].y, off));
+          const float2 oh = make_float2(__shfl_xor_sync(0xffffffffu, hi[c].x, off),
+                                        __shfl_xor_sync(0xffffffffu, hi[c].y, off));
+          const float2 ol = make_float2(__shfl_xor_sync(0xffffffffu, lo[c].x, off),
+                                        __shfl_xor_sync(0xffffffffu, lo[c].y, off));
           two_sum2(hi[c], lo[c], oh);
           lo[c] = __fadd2_rn(lo[c], ol);
         }
@@ -578,7 +584,8 @@ __global__ void __launch_bounds__(P2P32_WARPS * 32, 8) p2p_fp32_kernel(
           const double nq = -(double)tq[u];
           double v[4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) v[c] = u == 0 ? (double)hi[c].x + (double)lo[c].x : (double)hi[c].y + (double)lo[c].y;
+          for (int c = 0; c < 4; ++c)
+            v[c] = u == 0 ? (double)hi[c].x + (double)lo[c].x : (double)hi[c].y + (double)lo[c].y;
           out.add(j, v[0], nq * v[1], nq * v[2], nq * v[3]);
         }
       }
