@@ -1222,8 +1222,22 @@ b200fmm_status dense64_pairs(Context &c) {
   for (int t = 0; t < 343; ++t) largest = std::max<long long>(largest, s.h_first[t + 1] - s.h_first[t]);
   const size_t row = sizeof(double) * c.nn;
   size_t rows = std::max<size_t>((size_t)largest, std::min<size_t>((size_t)np * c.R, kDBytes / row));
-  bool ok = grow64(s.d_psrc, s.cap_psrc, (size_t)std::max<long long>(np, 1)) == B200FMM_OK &&
-            grow64(s.d_ppos, s.cap_ppos, (size_t)cells * 189) == B200FMM_OK;
+  // an eighth of the device stays free for what an evaluation cannot do without (a batch keeps many handles)
+  size_t avail = 0, device = 0;
+  const size_t nsrc = (size_t)std::max<long long>(np, 1), npos = (size_t)cells * 189;
+  auto more = [](size_t cap, size_t n, size_t bytes) { return n > cap ? (n - cap) * bytes : (size_t)0; };
+  const size_t tables = more(s.cap_psrc, nsrc, sizeof(int)) + more(s.cap_ppos, npos, sizeof(int));
+  auto fits = [&] {
+    const size_t need = tables + more(s.cap_d, rows * c.nn, sizeof(double));
+    if (need > 0 && device == 0) {
+      B200_CUDA(cudaMemGetInfo(&avail, &device));
+      avail -= std::min(avail, device / 8);
+    }
+    return need <= avail ? B200FMM_OK : B200FMM_ERR_OOM;
+  };
+  while (rows > (size_t)largest && fits() != B200FMM_OK) rows = std::max<size_t>((size_t)largest, rows / 2);
+  bool ok = fits() == B200FMM_OK && grow64(s.d_psrc, s.cap_psrc, nsrc) == B200FMM_OK &&
+            grow64(s.d_ppos, s.cap_ppos, npos) == B200FMM_OK;
   while (ok && s.cap_d < rows * c.nn && grow64(s.d_d, s.cap_d, rows * c.nn) != B200FMM_OK) {
     cudaGetLastError();
     if (rows == (size_t)largest) ok = false;

@@ -1114,6 +1114,36 @@ def test_pair_tables_are_for_whole_evaluations():
     f.close()
 
 
+@pytest.mark.parametrize("spare", [200 << 20, 2 << 20])  # the pairs' products in several chunks; the tile form
+def test_pair_tables_leave_an_eighth_of_the_device(spare):
+    """FP64 dense operators with little more than an eighth of the device free: the pairs' products (700 MB) take only
+    the rest.  With room again they are whole, and the results agree."""
+    torch = pytest.importorskip("torch")
+    n, height = 30000, 5
+    x, y, z = np.random.default_rng(9).random((3, n))
+    q = np.random.default_rng(10).uniform(-1, 1, n)
+    f = S.FMM("lagrange", 5, height)
+    f.set_particles(x, y, z, q)
+    f.synchronize()
+    free, device = torch.cuda.mem_get_info()
+    hold = torch.empty(free - device // 8 - spare, dtype=torch.uint8, device="cuda")
+    f.execute()
+    f.synchronize()
+    left = torch.cuda.mem_get_info()[0]
+    few = f.results()
+    del hold
+    torch.cuda.empty_cache()
+    assert left > device // 8 - (128 << 20)  # the tile form has 78 MB of partial sums
+    before = torch.cuda.mem_get_info()[0]
+    f.set_particles(x, y, z, q)
+    f.execute()
+    pairs = f.results()
+    assert before - torch.cuda.mem_get_info()[0] > 400 << 20
+    f.close()
+    for k in FIELDS:
+        assert S.rel_l2(few[k], pairs[k]) < 1e-12, k
+
+
 @pytest.mark.parametrize("kernel,precision,tol", [("cheb_sym", "fp64", 1e-12), ("cheb_sym", "mixed", 1e-10),
                                                   ("lagrange", "mixed", 1e-10)])
 def test_batch_matches_single_problems(kernel, precision, tol):
